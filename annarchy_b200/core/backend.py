@@ -18,10 +18,11 @@ Array names (the generated module binds a __constant__ pointer to each):
 from __future__ import annotations
 
 import numpy as np
+import scipy.sparse as sp
 
 from ..generator import formats as F
-from ..generator.codegen import (CodeGenerator, compensated_vars, global_equations, grid_for, list_grid,
-                                 trace_layout)
+from ..generator.codegen import (CodeGenerator, compensated_vars, global_equations, grid_for,
+                                 inbox_projections, list_grid, trace_layout)
 from ..runtime.lib import DryNative, NativeNet
 from .monitor import array_name
 
@@ -65,6 +66,8 @@ class CompiledNetwork:
         self.shard = net._config.get("shard")
         self.owned: dict[int, tuple[int, int]] = {}
         self._exchange = None
+        # projections delivered through per-neuron inboxes (double precision)
+        self.inbox: set = set()
 
     # --------------------------------------------------------------- helpers
     def _w(self, w: np.ndarray) -> np.ndarray:
@@ -120,6 +123,7 @@ class CompiledNetwork:
         self.spike_lists = (not self.exact and self.engine == "grid" and not self.shard)
         if self.shard:
             self._setup_shard()
+        self.inbox = inbox_projections(self)
         for pop in net.populations:
             self._create_population(pop)
         for proj in net.projections:
@@ -137,6 +141,7 @@ class CompiledNetwork:
             mod = gen.local_module()
         else:
             nat.create("tickc", np.zeros(1, dtype=np.uint32))
+            nat.create("tstep", np.zeros(1, dtype=np.int64))
             if any(getattr(p, "stop_condition", None) for p in net.populations):
                 nat.create("stop_flags", np.full(len(net.populations), -1, dtype=np.int64))
             if self._persistent() and gen.persistent_ok():
@@ -474,7 +479,6 @@ class CompiledNetwork:
                 for suffix in ("__post_rank", "__row_ptr", "__col", "__w"):
                     nat.free(f"proj{k}{suffix}")
                 proj._device_conn = None
-                import scipy.sparse as sp
                 proj._store(sp.csr_matrix((w, col, rp), shape=(npost, npre)), d["name"],
                             d["storage_format"], d["delays"])
                 return self._create_projection(proj)
@@ -529,15 +533,16 @@ class CompiledNetwork:
         for prm in proj.desc["parameters"] + proj.desc["variables"]:
             if prm["locality"] == "global":
                 nat.create(f"proj{k}__{prm['name']}", np.array([prm["init"]], dtype=self.real))
-        if not self.exact:
-            nat.csr_to_csc(f"proj{k}", proj.pre_pop.size, with_weights=not plastic)
+        if not self.exact or k in self.inbox:
+            nat.csr_to_csc(f"proj{k}", proj.pre_pop.size, with_weights=not plastic and not self.exact)
         mean_fan = nnz / max(1, pre_hi - pre_lo)
         lay["chunks"] = max(1, -(-int(1.25 * mean_fan) // 32))
         lay["post_chunks"] = max(1, -(-int(lengths.max() if lengths.size else 1) // 32))
-        if plastic and self.spike_lists:
+        if plastic or k in self.inbox:
             row_of = np.full(proj.post_pop.size, -1, dtype=np.int32)
             row_of[post0:post0 + npost] = np.arange(npost, dtype=np.int32)
             nat.create(f"proj{k}__row_of", row_of)
+        self._create_inbox(proj, nnz)
         if self.spike_lists:
             lay["grid"] = list_grid(pre_hi - pre_lo, lay["chunks"])
         elif self.exact or plastic:
@@ -563,6 +568,22 @@ class CompiledNetwork:
                 nat.create_empty(f"proj{k}___last_event", np.int64, (nnz,))
                 nat.fill(f"proj{k}___last_event", np.int64(-10000))
         self.layout[k] = lay
+
+    def _create_inbox(self, proj, nnz):
+        """Inbox of every post neuron (counter, entries), the copy of the
+        bitmap words its row walk reads and, for plastic synapses, the value
+        each one transmitted (see anb_inbox_add)."""
+        k = proj.id
+        if k not in self.inbox:
+            return
+        nat = self.native
+        n = proj.post_pop.size
+        key = np.uint64 if proj._delay_steps is not None else np.uint32
+        nat.create(f"proj{k}__ibn", np.zeros(n, dtype=np.uint32))
+        nat.create_empty(f"proj{k}__ibx", key, (n * 8,))
+        nat.create(f"proj{k}__ibb", np.zeros((proj.pre_pop.size + 31) // 32, dtype=np.uint32))
+        if proj.plastic:
+            nat.create_empty(f"proj{k}__pv", np.float64, (nnz,))
 
     def _create_delays(self, proj):
         k = proj.id
@@ -705,24 +726,26 @@ class CompiledNetwork:
             # pre-major view (the reference's CSRC column view, CSRCMatrix.hpp:164-222)
             npre = proj.pre_pop.size
             rows_of = np.repeat(np.arange(rows, dtype=np.int64), np.diff(row_ptr))
-            order = np.lexsort((rows_of, cols))
+            # synapses by pre rank, then row: a counting sort (scipy's transposition)
+            order = sp.csr_matrix((np.arange(nnz), cols, row_ptr), shape=(rows, npre)).tocsc().data
             col_ptr = np.zeros(npre + 1, dtype=np.int32)
             np.cumsum(np.bincount(cols, minlength=npre), out=col_ptr[1:])
             nat.create(f"proj{k}__col_ptr", col_ptr)
             self._col_ptr[k] = col_ptr
             nat.create(f"proj{k}__post_idx", post_rank[rows_of[order]].astype(np.int32))
             nat.create(f"proj{k}__inv_idx", order.astype(np.int32))
-            if not proj.plastic:
-                nat.create(f"proj{k}__w_pre", self._w(w[order]) if not self.exact else w[order])
+            if not proj.plastic and not self.exact:
+                nat.create(f"proj{k}__w_pre", self._w(w[order]))
             lay["w0"] = int(proj.pre_ranks.min()) // 32
             lay["w1"] = int(proj.pre_ranks.max()) // 32 + 1
             fan = np.diff(col_ptr)
             lay["chunks"] = max(1, -(-int(fan.max() if fan.size else 1) // 32))
             lay["post_chunks"] = max(1, -(-int(np.diff(row_ptr).max() if rows else 1) // 32))
-            if proj.plastic and self.spike_lists:
+            if proj.plastic or k in self.inbox:
                 row_of = np.full(proj.post_pop.size, -1, dtype=np.int32)
                 row_of[post_rank] = np.arange(rows, dtype=np.int32)
                 nat.create(f"proj{k}__row_of", row_of)
+            self._create_inbox(proj, nnz)
             # warp per post row: exact order, per-synapse delays, and plastic
             # delayed projections (the spike lists hold only the last step)
             gather = self.exact or proj._delay_steps is not None or (

@@ -40,9 +40,24 @@ extern "C" __global__ void check_spike_gather(int n, const int* rp, const int* c
                                               const anb_u32* spk, const int* pr, double* g) {
   anb_spike_gather<double, double>(n, rp, c, w, spk, pr, g);
 }
+extern "C" __global__ void check_inbox(const anb_u32* spk, const int* cp, const int* pi, const int* ii,
+                                       const int* rp, const int* c, const double* w, const int* d,
+                                       anb_u32* cnt, unsigned* ent, unsigned long long* entd, double* g) {
+  __shared__ int list[4 * ANB_DELIVER_LIST + 1];
+  const int n = anb_list_spikes(list, spk, 8, 0, 8, 4, 9, 32 * blockIdx.x, 32, cp, nullptr);
+  anb_for_spikes(list, n, [&](const int, const int dd, const int q) {
+                   anb_inbox_put(cnt, ent, pi[q], (unsigned)ii[q]);
+                   anb_inbox_put(cnt, entd, pi[q], (unsigned long long)dd << 32 | (unsigned)ii[q]);
+                 });
+  const int i = threadIdx.x;
+  double s = anb_inbox_add(g[i], cnt[i], ent, i, w);
+  s = anb_inbox_add(s, cnt[i], entd, i, w);
+  s = anb_row_gather<double>(s, rp[0], rp[1], c, w, spk);
+  g[i] = anb_row_gather_delayed<double>(s, rp[0], rp[1], c, w, d, spk, spk, 8, 4, 9);
+}
 extern "C" __global__ void check_spike_scatter(const anb_u32* spk, const int* cp, const int* pi,
                                                const anb_bf16* w, float* g) {
-  anb_spike_scatter<float, anb_bf16>(0, 128, spk, cp, pi, w, g);
+  anb_spike_scatter<float, anb_bf16>(0, 128, spk, cp, pi, w, g, blockIdx.x, gridDim.x);
 }
 extern "C" __global__ void __launch_bounds__(384, 3) check_rate_pcsr_f32(
     const int* cp, const int* wt, const unsigned short* c, const float* w, const float* x, int n_pre,
