@@ -23,6 +23,7 @@ import scipy.sparse as sp
 from ..generator import formats as F
 from ..generator.codegen import (CodeGenerator, compensated_vars, global_equations, grid_for,
                                  inbox_projections, list_grid, trace_layout)
+from ..generator.resident import Resident, possible as resident_possible
 from ..runtime.lib import DryNative, NativeNet
 from .monitor import array_name
 
@@ -124,6 +125,7 @@ class CompiledNetwork:
         if self.shard:
             self._setup_shard()
         self.inbox = inbox_projections(self)
+        resident = self._resident_layout()
         for pop in net.populations:
             self._create_population(pop)
         for proj in net.projections:
@@ -134,6 +136,14 @@ class CompiledNetwork:
             pop._init_state = {k: v.copy() for k, v in pop._host.items()}
         if self.engine == "local":
             self._build_cluster()
+            return
+        if resident:
+            res, lay = resident
+            res.create_arrays(lay)
+            self.module = res.module(lay)
+            nat.load_module(self.module.source, self.module.options)
+            self.write_constants()
+            nat.set_local_kernel(*self.module.local)
             return
         gen = CodeGenerator(self)
         if self.engine == "local":
@@ -160,6 +170,20 @@ class CompiledNetwork:
             nat.set_pdl(bool(net._config.get("pdl", True)))
             for pop_id, kernel, grid, block, mode_all in mod.stops:
                 nat.set_stop_kernel(pop_id, kernel, grid, block, mode_all)
+
+    def _resident_layout(self):
+        """(Resident, layout) of a rate-coded network that stays on chip for a
+        whole run (engine "auto"), which then becomes the engine."""
+        if self.engine != "grid" or self.net._config.get("engine", "auto") != "auto":
+            return None
+        if not resident_possible(self):
+            return None
+        res = Resident(self)
+        lay = res.choose()
+        if lay is None:
+            return None
+        self.engine = "resident"
+        return res, lay
 
     def _persistent(self) -> bool:
         """Run the grid engine's step as one persistent cooperative launch
@@ -704,7 +728,8 @@ class CompiledNetwork:
                 for name, arr in proj._host_semi.items():
                     nat.create(f"proj{k}__{name}", np.asarray(arr, dtype=self.real))
                 nat.create(f"proj{k}__flags", np.array(proj._learn_flags, dtype=np.int32))
-            fmt = ("csr" if (proj._delay_steps is not None or learning or custom)
+            fmt = ("csr" if (proj._delay_steps is not None or learning or custom
+                             or self.engine == "resident")
                    else self._rate_format(proj, lay))
             lay["format"] = fmt
             if fmt != "csr":

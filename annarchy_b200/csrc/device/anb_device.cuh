@@ -1268,6 +1268,131 @@ __device__ __forceinline__ bool anb_grid_sync(unsigned* bar, int* err) {
   return anb_gs_ok != 0;
 }
 
+// ---- rate-coded networks that stay on chip -------------------------------------------------
+// A CTA keeps the incoming synapses of its neurons in shared memory, as items
+// of ROWS rows (one warp at a time) with LANES lanes per row: step m of an
+// item holds element m * LANES + g of row q at position q * LANES + g, so a
+// warp's loads of weights and columns are conflict-free; the rates are
+// gathered from the CTA's copy. What bounds a step: in double precision the
+// chain of ordered additions of a row (the loads of UNROLL steps are issued
+// ahead of it), the exchange of the rates and the barrier.
+
+// Fills a projection's part of the CTA's pool: rb = (first element of the part
+// in ri, its elements, its place in the pool), ri = each element's place in
+// the CSR arrays; -1 (past a row's end) gets weight 0 and column `pad`, where
+// the CTA's copy of the rates holds a zero.
+template <typename W>
+__device__ __noinline__ void anb_rate_fill(const int* __restrict__ rb, const int* __restrict__ ri,
+                                              const int* __restrict__ col, const W* __restrict__ w,
+                                              int pad, W* pool_w, unsigned short* pool_c) {
+  const int* __restrict__ src = ri + rb[0];
+  const int n = rb[1], at = rb[2];
+#pragma unroll 2
+  for (int k = threadIdx.x; k < n; k += blockDim.x) {
+    const int j = src[k];
+    pool_w[at + k] = j >= 0 ? w[j] : W(0);
+    pool_c[at + k] = (unsigned short)(j >= 0 ? col[j] : pad);
+  }
+}
+
+// Loads from shared-memory addresses (volatile: not moved across barriers).
+__device__ __forceinline__ void anb_lds(unsigned a, float* v) {
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(*v) : "r"(a));
+}
+__device__ __forceinline__ void anb_lds(unsigned a, double* v) {
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(*v) : "r"(a));
+}
+__device__ __forceinline__ void anb_lds(unsigned a, unsigned short* v) {
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(*v) : "r"(a));
+}
+
+// Weighted sum of the calling lane's row of one item (all lanes of the row
+// get it; whole warp): blocks of U steps, the columns loaded two blocks and
+// the rates and weights one block ahead of the additions. Double precision:
+// one lane, stored order, bound by the chain of additions (9 cycles each); a
+// padding element adds +0, which changes no sum. The columns' loads may run
+// two blocks past the item (inside the CTA's pool, which is that much longer).
+// Pool and rates as shared-memory addresses; not inlined (a network calls it
+// once per projection, and its code is most of the module's compile time).
+template <typename R, typename W, int LANES, int ROWS>
+__device__ __noinline__ R anb_rate_row(int first, int steps, unsigned pool_w, unsigned pool_c, unsigned x) {
+  constexpr int U = LANES == 1 ? 8 : 4, L = ROWS * LANES;
+  const int lane = threadIdx.x & 31;
+  const int at = first + (lane < L ? lane : 0);
+  unsigned w = pool_w + (unsigned)(at * sizeof(W)), c = pool_c + 2u * at;
+  R s = R(0), p[U];
+  if (steps > 0) {
+    unsigned short cn[U];
+    R xn[U];
+    W wn[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) anb_lds(c + 2u * u * L, &cn[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      anb_lds(x + (unsigned)sizeof(R) * cn[u], &xn[u]);
+      anb_lds(w + (unsigned)sizeof(W) * u * L, &wn[u]);
+      anb_lds(c + 2u * (U + u) * L, &cn[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) p[u] = xn[u] * (R)anb_wf(wn[u]);
+#pragma unroll 1
+    for (int m = U; m < steps; m += U) {
+      w += (unsigned)sizeof(W) * U * L;
+      c += 2u * U * L;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        anb_lds(x + (unsigned)sizeof(R) * cn[u], &xn[u]);
+        anb_lds(w + (unsigned)sizeof(W) * u * L, &wn[u]);
+        anb_lds(c + 2u * (U + u) * L, &cn[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) s += p[u];
+#pragma unroll
+      for (int u = 0; u < U; ++u) p[u] = xn[u] * (R)anb_wf(wn[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) s += p[u];
+  }
+#pragma unroll
+  for (int o = LANES / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+__device__ __forceinline__ void anb_cluster_st(unsigned addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void anb_cluster_st(unsigned addr, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+
+// Grid-wide barrier on a counter that only grows (zero at the launch): the
+// CTA's arrival, then a bounded wait until `target` arrivals. Returns false
+// when this or another CTA gave up (see anb_grid_sync).
+__device__ __forceinline__ bool anb_grid_meet(unsigned* bar, unsigned target, int* err) {
+  __shared__ int anb_gm_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    // the release covers the CTA's writes: the CTA barrier orders them before it
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    int ok = 1;
+    unsigned v = 0;
+    const long long c0 = clock64();
+    for (int it = 0;; ++it) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      if ((int)(v - target) >= 0) break;
+      if ((it & 63) == 63 && (clock64() - c0 > ANB_GRID_WAIT_CYCLES ||
+                              *(volatile int*)err == ANB_DEVERR_BARRIER_TIMEOUT)) {
+        ok = 0;
+        break;
+      }
+    }
+    if (!ok) atomicExch(err, ANB_DEVERR_BARRIER_TIMEOUT);
+    anb_gm_ok = ok;
+  }
+  __syncthreads();
+  return anb_gm_ok != 0;
+}
+
 // ---- monitors ---------------------------------------------------------------------------
 
 // Copy n values (converted to double) into slot `slot` of a ring of `cap` slots.

@@ -40,6 +40,16 @@ extern "C" __global__ void check_spike_gather(int n, const int* rp, const int* c
                                               const anb_u32* spk, const int* pr, double* g) {
   anb_spike_gather<double, double>(n, rp, c, w, spk, pr, g);
 }
+extern "C" __global__ void __launch_bounds__(512, 1) check_resident(const int* rb, const int* ri, const int* c,
+                                                                  const double* w, double* x, unsigned* bar,
+                                                                  int* err) {
+  __shared__ double pw[1024];
+  __shared__ unsigned short pc[1024];
+  anb_rate_fill(rb, ri, c, w, 7, pw, pc);
+  if (!anb_grid_meet(bar, 1u, err)) return;
+  x[threadIdx.x] = anb_rate_row<double, double, 1, 32>(rb[0], rb[1], anb_smem_addr(pw), anb_smem_addr(pc), 0u);
+  anb_cluster_st(anb_cluster_map(anb_smem_addr(pw), 0u), 1.0);
+}
 extern "C" __global__ void check_inbox(const anb_u32* spk, const int* cp, const int* pi, const int* ii,
                                        const int* rp, const int* c, const double* w, const int* d,
                                        anb_u32* cnt, unsigned* ent, unsigned long long* entd, double* g) {
