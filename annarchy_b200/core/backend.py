@@ -23,6 +23,7 @@ import scipy.sparse as sp
 from ..generator import formats as F
 from ..generator.codegen import (CodeGenerator, compensated_vars, global_equations, grid_for,
                                  inbox_projections, list_grid, trace_layout)
+from ..generator.masks import Masks
 from ..generator.resident import Resident, possible as resident_possible
 from ..runtime.lib import DryNative, NativeNet
 from .monitor import array_name
@@ -198,6 +199,19 @@ class CompiledNetwork:
         synapses; otherwise 8 CTAs with the synapses read from global memory.
         A cluster the device cannot schedule falls back the same way."""
         from ..runtime.lib import BackendError
+        masks = Masks(self)
+        for lay in masks.choose() if masks.possible() else []:
+            masks.create_arrays(lay)
+            mod = masks.module(lay)
+            try:
+                self.native.load_module(mod.source, mod.options)
+                self.write_constants()
+                self.native.set_local_kernel(*mod.local)
+            except BackendError:
+                continue                       # a cluster the device cannot schedule
+            self.module = mod
+            self.engine = "cluster"
+            return
         want = self.net._config.get("cluster_size")
         total = max(p.size for p in self.net.populations)
         cands = [int(want)] if want else [c for c in (1, 2, 4, 8, 16) if (total + c - 1) // c <= 1024]

@@ -1205,6 +1205,70 @@ __device__ __forceinline__ void anb_cluster_sync() {
                    : "memory");
 }
 
+// mbarriers of this CTA (shared-memory addresses): `count` arrivals per phase,
+// one of them with the bytes to expect from the cluster's other CTAs.
+__device__ __forceinline__ void anb_mbar_init(unsigned bar, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ void anb_mbar_expect(unsigned bar, unsigned bytes) {
+  asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }"
+               ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void anb_mbar_arrive(unsigned bar) {
+  asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(bar) : "memory");
+}
+// Bounded wait (about a second) for the phase of the given parity; false and
+// an error code when it ran out. Polls without suspending: the phases are a
+// few hundred cycles apart.
+__device__ __forceinline__ bool anb_mbar_wait(unsigned bar, unsigned parity, int* err) {
+  unsigned done = 0;
+  long long c0 = 0;
+  for (int it = 1;; ++it) {
+    asm volatile(
+        "{ .reg .pred p; mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    if (done) return true;
+    if ((it & 1023) == 0) {
+      const long long c = clock64();
+      if (c0 == 0) c0 = c;
+      if (c - c0 > 2000000000ll) {
+        anb_report(err, ANB_DEVERR_BARRIER_TIMEOUT);
+        return false;
+      }
+    }
+  }
+}
+
+// Appends the values v of the lanes with `in` to a list of *n entries.
+__device__ __forceinline__ void anb_pack(anb_u32 v, bool in, anb_u32* list, int* n) {
+  const unsigned z = __ballot_sync(0xffffffffu, in);
+  if (in) list[*n + __popc(z & ((1u << (threadIdx.x & 31)) - 1u))] = v;
+  *n += __popc(z);
+}
+// g plus w once for every one of the n listed masks with this lane's bit (the
+// list is 16-byte aligned and padded to a multiple of 4 with zeros).
+template <typename R>
+__device__ __forceinline__ R anb_mask_add(R g, R w, const anb_u32* list, int n) {
+  const anb_u32 bit = 1u << (threadIdx.x & 31);
+#pragma unroll 1
+  for (int k = 0; k < n; k += 4) {
+    const uint4 v = *reinterpret_cast<const uint4*>(list + k);
+    if (v.x & bit) g += w;
+    if (v.y & bit) g += w;
+    if (v.z & bit) g += w;
+    if (v.w & bit) g += w;
+  }
+  return g;
+}
+// Store of one word into another CTA of the cluster, counted on that CTA's
+// mbarrier (launches with a cluster only; the own CTA's word is an ordinary
+// store).
+__device__ __forceinline__ void anb_st_async(unsigned addr, anb_u32 v, unsigned bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.u32 [%0], %1, [%2];"
+               ::"r"(addr), "r"(v), "r"(bar) : "memory");
+}
+
 // Fast scatter from a spike list: work item = (spike, 32-synapse chunk of its
 // fan-out), so a warp does one pass per item whatever the fan-out; spikes
 // outside [lo, hi) (not pre neurons of this projection) are skipped.

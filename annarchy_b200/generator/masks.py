@@ -1,0 +1,323 @@
+"""Small spiking networks on one thread-block cluster, every warp on its own.
+
+CTA r owns the neurons [r * chunk, (r + 1) * chunk) of every population, a
+warp 32 of them, a lane one, whose state stays in registers for a whole run.
+The CTA's shared memory holds, per pre-synaptic neuron and warp, a 32-bit mask
+of the lanes it has a synapse on; all synapses of a projection carry one
+weight. A step of a warp:
+
+  1. wait until every warp's spikes of the previous step have arrived in this
+     CTA's copy of the spike bitmaps (an mbarrier counting the bytes from the
+     other CTAs and one arrival per own warp);
+  2. every lane takes a few words of the bitmap and loads the mask of the spike
+     it finds; the masks that are not empty are packed into a short list per
+     projection (a second round takes the second spikes of the words, and so
+     on), and every lane adds the projection's weight once per listed mask with
+     its bit. The reference adds them in ascending pre rank (ANNarchy/generator/
+     Projection/OpenMP/CSR.py:870-902): with one weight per projection that is
+     the same sequence of additions;
+  3. update its neurons, store the ballot of the new spikes in the own copy
+     and send it to every other CTA (st.async: the bytes land and are counted
+     in one trip).
+
+No CTA or cluster barrier in the loop: a warp that has received all words of
+step s knows that every warp has finished reading those of step s - 1, so two
+copies of the bitmaps (by step parity) are enough. What bounds a step is this
+chain, and the instructions of eight warps per SM: the control flow is
+uniform, since forms in which the warp went through the spikes one after
+another (100 cycles per spike), lanes looped over their own spikes (shared-
+memory counters: 1000 cycles) or one warp listed them for the CTA were slower.
+
+Measured per step against the form with a cluster barrier per step and the
+synapses listed per pre-synaptic neuron (CodeGenerator.cluster_module, which
+remains for projections with several weights and for larger populations): 4000
+neurons, 8 spikes per step 1.19 us (2.56) in double and 0.99 us (1.69) in single
+precision; 1000 neurons 0.66 and 0.46 us; 400 neurons 0.62 and 0.44 us.
+"""
+from __future__ import annotations
+
+import re
+
+import numpy as np
+
+from .codegen import CodeGenerator, Module, compensated_vars
+
+SMEM_LIMIT = 220 * 1024
+MAX_WORDS = 256            # bitmap words of a population (8 per lane)
+
+
+class Masks:
+    def __init__(self, c):
+        self.c = c
+        self.net = c.net
+
+    def possible(self) -> bool:
+        """One weight per projection, populations of up to 8192 neurons."""
+        net = self.net
+        if any((p.size + 31) // 32 > MAX_WORDS for p in net.populations):
+            return False
+        for p in net.projections:
+            d = p._csr.data
+            if d.size and not np.all(d == d[0]):
+                return False
+        return True
+
+    def slots(self):
+        """Projections grouped into mask tables: one joins the table before it
+        when both populations are the same and their pre-synaptic words are
+        disjoint. Tables keep the projections' order."""
+        out = []
+        for p in self.net.projections:
+            lay = self.c.layout[p.id]
+            w0, w1 = lay["w0"], lay["w1"]
+            if out:
+                s = out[-1]
+                if s["pre"] is p.pre_pop and s["post"] is p.post_pop and all(
+                        w1 <= a or b <= w0 for _, a, b in s["projs"]):
+                    s["projs"].append((p, w0, w1))
+                    s["w0"], s["w1"] = min(s["w0"], w0), max(s["w1"], w1)
+                    continue
+            out.append({"pre": p.pre_pop, "post": p.post_pop, "projs": [(p, w0, w1)], "w0": w0, "w1": w1})
+        return out
+
+    def layout(self, C: int):
+        """Shared memory of a CTA of a C-CTA cluster, or None."""
+        a16 = lambda x: (int(x) + 15) // 16 * 16
+        off, lay = 64, {"pop": {}, "slots": self.slots()}             # two mbarriers first
+        for pop in self.net.populations:
+            chunk = -(-(-(-pop.size // C)) // 32) * 32
+            words = (pop.size + 31) // 32
+            per = -(-words // 32)                                     # words a lane takes
+            d = {"chunk": chunk, "words": words, "per": per, "rep": []}
+            for _ in (0, 1):
+                d["rep"].append(off)
+                off += a16(per * 32 * 4)
+            lay["pop"][pop.id] = d
+        lay["block"] = max(d["chunk"] for d in lay["pop"].values())
+        if lay["block"] > 1024:
+            return None
+        # no CTA without neurons: one that sends nothing would not be waited for
+        lay["C"] = max(-(-p.size // lay["pop"][p.id]["chunk"]) for p in self.net.populations)
+        for s in lay["slots"]:
+            s["warps"] = lay["pop"][s["post"].id]["chunk"] // 32
+            s["rows"] = (s["w1"] - s["w0"]) * 32
+            s["off"], off = off, off + a16(s["rows"] * s["warps"] * 4)
+            # per warp and projection, the masks of one round
+            s["cap"] = lay["pop"][s["pre"].id]["per"] * 32 + 4
+            s["list"], off = off, off + 4 * s["cap"] * len(s["projs"]) * s["warps"]
+        lay["smem"] = off
+        return lay if off <= SMEM_LIMIT else None
+
+    def choose(self):
+        """Layouts to try, the preferred one first: about 128 neurons per CTA
+        (four warps: one per scheduler), at most 16 CTAs. 1000 neurons on 1, 2,
+        4, 8 and 16 CTAs: 1.37, 0.82, 0.70, 0.66, 0.69 us per step in double."""
+        want = self.net._config.get("cluster_size")
+        if want:
+            lays = [self.layout(int(want))]
+        else:
+            total = max(p.size for p in self.net.populations)
+            first = next((c for c in (1, 2, 4, 8) if total <= 128 * c), 16)
+            lays = [self.layout(c) for c in (1, 2, 4, 8, 16) if c >= first]
+        return [x for x in lays if x]
+
+    def tables(self, slot, lay):
+        """(C x rows x warps) masks of a table."""
+        chunk, W, rows = lay["pop"][slot["post"].id]["chunk"], slot["warps"], slot["rows"]
+        m = np.zeros(lay["C"] * rows * W)
+        for proj, _, _ in slot["projs"]:
+            post_rank, row_ptr, cols, _ = proj.csr_population_ranks()
+            post = np.repeat(post_rank, np.diff(row_ptr)).astype(np.int64)
+            q = post % chunk
+            idx = ((post // chunk) * rows + (cols - 32 * slot["w0"])) * W + (q >> 5)
+            m += np.bincount(idx, weights=np.ldexp(1.0, (q & 31).astype(np.int32)), minlength=m.size)
+        return m.astype(np.uint32)
+
+    def create_arrays(self, lay):
+        nat = self.c.native
+        for i, s in enumerate(lay["slots"]):
+            nat.create(f"net__masks{i}", self.tables(s, lay))
+            for proj, _, _ in s["projs"]:
+                w = proj._csr.data
+                nat.create(f"proj{proj.id}__mw", self.c._w(np.array([w[0] if w.size else 0.0])))
+
+    def module(self, lay) -> Module:
+        c, net = self.c, self.net
+        gen = CodeGenerator(c)
+        R, C, block = gen.real, lay["C"], lay["block"]
+        regs, load, store, ranges, ups, deliver, words_sent = [], [], [], [], [], "", 0
+        for pop in net.populations:
+            k, d = pop.id, lay["pop"][pop.id]
+            words_sent += d["words"]
+            ranges += [f"const int anb_base{k} = (int)anb_rank * {d['chunk']};",
+                       f"const int anb_cnt{k} = max(0, min({pop.size} - anb_base{k}, {d['chunk']}));",
+                       f"anb_u32* const anb_rep{k}0 = reinterpret_cast<anb_u32*>(anb_smem + {d['rep'][0]});",
+                       f"anb_u32* const anb_rep{k}1 = reinterpret_cast<anb_u32*>(anb_smem + {d['rep'][1]});"]
+            spk = gen.ptr(f"pop{k}__spk")
+            load.append(f"#pragma unroll 1\n    for (int q = threadIdx.x; q < {32 * d['per']}; q += {block}) {{ "
+                        f"anb_rep{k}1[q] = q < {d['words']} ? {spk}[q] : 0u; anb_rep{k}0[q] = 0u; }}")
+            store.append(f"if (anb_tid < anb_cnt{k} && anb_lane == 0) {spk}[(anb_base{k} + anb_tid) >> 5] = "
+                         f"(nsteps & 1 ? anb_rep{k}0 : anb_rep{k}1)[(anb_base{k} + anb_tid) >> 5];")
+            smem = {}
+            names = [(n, R) for n in c._local_vars(pop)] + [("refractory_remaining", "int")]
+            if pop._has_refractory:
+                names.append(("refractory", "int"))
+            names += [("kc_" + n, R) for n in compensated_vars(pop, c.exact, net._config)]
+            for n, ct in names:
+                reg = f"anb_rg{k}_{n}"
+                smem[n] = reg
+                regs.append(f"{ct} {reg} = ({ct})0;")
+                if n.startswith("kc_"):
+                    continue
+                g = gen.ptr(f"pop{k}__{n}")
+                load.append(f"if (anb_tid < anb_cnt{k}) {reg} = {g}[anb_base{k} + anb_tid];")
+                if n != "refractory":
+                    store.append(f"if (anb_tid < anb_cnt{k}) {g}[anb_base{k} + anb_tid] = {reg};")
+            ups.append(self._update(gen, pop, smem, lay))
+        for i, s in enumerate(lay["slots"]):
+            a, b = s["pre"].id, s["post"].id
+            per = lay["pop"][a]["per"]
+            n4 = s["rows"] * s["warps"]
+            load.append(f"#pragma unroll 4\n    for (int q = threadIdx.x; q < {n4}; q += {block}) "
+                        f"reinterpret_cast<anb_u32*>(anb_smem + {s['off']})[q] = "
+                        f"{gen.ptr(f'net__masks{i}')}[(size_t)anb_rank * {n4} + q];")
+            regs.append(f"const anb_u32* const anb_mask{i} = reinterpret_cast<const anb_u32*>(anb_smem + {s['off']}) + anb_warp;")
+            regs.append(f"anb_u32* const anb_li{i} = reinterpret_cast<anb_u32*>(anb_smem + {s['list']}) + "
+                        f"anb_warp * {s['cap'] * len(s['projs'])};")
+            pack, adds = "", ""
+            for q, (proj, w0, w1) in enumerate(s["projs"]):
+                regs.append(f"const {R} anb_w{proj.id} = ({R})anb_wf({gen.ptr(f'proj{proj.id}__mw')}[0]);")
+                at = f"anb_li{i} + {q * s['cap']}"
+                pack += f"""
+            int anb_n{q} = 0;"""
+                for j in range(w0 // 32, (w1 - 1) // 32 + 1):
+                    # (words outside the projection's range belong to others)
+                    inside = "" if w0 <= 32 * j and 32 * j + 32 <= w1 else \
+                        f" && anb_lane >= {max(0, w0 - 32 * j)} && anb_lane < {min(32, w1 - 32 * j)}"
+                    pack += f"""
+            anb_pack(anb_m[{j}], anb_m[{j}] != 0u{inside}, {at}, &anb_n{q});"""
+                pack += f"""
+            if (anb_lane < 4) ({at})[anb_n{q} + anb_lane] = 0u;"""
+                adds += f"""
+            anb_rg{b}_g_{proj.target} = anb_mask_add(anb_rg{b}_g_{proj.target}, anb_w{proj.id}, {at}, anb_n{q});  // {proj.name}"""
+            word = "anb_rep[j * 32 + anb_lane]"
+            used = [(w0, w1) for _, w0, w1 in s["projs"]]
+            if len(used) != 1 or used[0] != (0, lay["pop"][a]["words"]):
+                word = " || ".join(f"(j * 32 + anb_lane >= {w0} && j * 32 + anb_lane < {w1})"
+                                   for w0, w1 in used) + " ? " + word + " : 0u"
+            any_x = " | ".join(f"anb_x[{j}]" for j in range(per))
+            deliver += f"""
+        if (anb_warp < {s['warps']}) {{  // population {a}'s spikes of the previous step (word j * 32 + lane: lane's j-th)
+          const anb_u32* anb_rep = (anb_s & 1) ? anb_rep{a}0 : anb_rep{a}1;
+          anb_u32 anb_x[{per}], anb_m[{per}];
+#pragma unroll
+          for (int j = 0; j < {per}; ++j) anb_x[j] = {word};
+#pragma unroll 1
+          while (__any_sync(0xffffffffu, ({any_x}) != 0u)) {{
+            // the mask of each word's first spike
+#pragma unroll
+            for (int j = 0; j < {per}; ++j) {{
+              anb_m[j] = anb_x[j] ? anb_mask{i}[((j * 32 + anb_lane) * 32 + __ffs(anb_x[j]) - {s['w0'] * 32 + 1}) * {s['warps']}] : 0u;
+              anb_x[j] &= anb_x[j] - 1u;
+            }}{pack}
+            __syncwarp();{adds}
+            __syncwarp();
+          }}
+        }}"""
+        globals_ = [gen._globals_preamble(p, lambda n, kk=p.id: gen.ptr(f"pop{kk}__{n}")) for p in net.populations]
+        mon_pre = "\n    ".join(
+            f"const int anb_mon_on{m.id} = {gen.ptr(f'mon{m.id}__on')}[0];\n    "
+            f"const long long anb_sl{m.id} = t0 - {gen.ptr(f'mon{m.id}__t0')}[0];\n    "
+            f"const int anb_slot0{m.id} = anb_sl{m.id} < -(1 << 30) || anb_sl{m.id} > (1 << 30) ? -(1 << 30) : (int)anb_sl{m.id};"
+            for m in net.monitors)
+        dt_t = "double" if c.exact else "float"
+        warps = f"anb_cnt{net.populations[0].id}"
+        for p in net.populations[1:]:
+            warps = f"max({warps}, anb_cnt{p.id})"
+        own = " + ".join(f"(anb_cnt{p.id} + 31) / 32" for p in net.populations)
+        nl = "\n    "
+        err = gen.ptr("err")
+        src = f"""
+extern "C" __global__ void __launch_bounds__({block}, 1) anb_cluster_run(long long t0, int nsteps) {{
+    extern __shared__ __align__(16) unsigned char anb_smem[];
+    const unsigned anb_rank = anb_cluster_rank();
+    const {dt_t} dt = ({dt_t})(*{gen.ptr('dt')});
+    const int anb_tid = threadIdx.x, anb_lane = threadIdx.x & 31, anb_warp = threadIdx.x >> 5;
+    // mbarriers: the words of even and of odd steps
+    const unsigned anb_bar = anb_smem_addr(anb_smem);
+    {nl.join(ranges)}
+    // lane c: CTA c's shared memory (the mbarriers at its start)
+    const unsigned anb_peer = anb_cluster_map(anb_bar, anb_lane < {C} ? anb_lane : 0);
+    (void)anb_peer;
+    const int anb_warps = ({warps} + 31) / 32;
+    const unsigned anb_bytes = 4u * ({words_sent} - ({own}));
+    {nl.join(regs)}
+    {nl.join(g for g in globals_ if g)}
+    {mon_pre}
+    if (threadIdx.x == 0) {{
+      // a phase: thread 0 (the bytes to expect) and every warp with neurons
+      anb_mbar_init(anb_bar, 1 + anb_warps);
+      anb_mbar_init(anb_bar + 8, 1 + anb_warps);
+      anb_mbar_expect(anb_bar, anb_bytes);
+      anb_mbar_expect(anb_bar + 8, anb_bytes);
+    }}
+    {nl.join(load)}
+    anb_cluster_sync();
+    // (warps without neurons send nothing, so nobody waits for them: they stay out)
+    if (anb_warp < anb_warps) {{
+#pragma unroll 1
+      for (int anb_s = 0; anb_s < nsteps; ++anb_s) {{
+        const long long t = t0 + anb_s;
+        if (anb_s > 0) {{
+          // the words of step s - 1; the barrier's next phase takes those of s + 1
+          const unsigned b = anb_bar + 8u * ((anb_s - 1) & 1);
+          if (!anb_mbar_wait(b, ((anb_s - 1) >> 1) & 1, {err})) break;
+          if (threadIdx.x == 0) anb_mbar_expect(b, anb_bytes);
+        }}{deliver}
+        {''.join(ups)}
+        __syncwarp();
+        if (anb_lane == 0) anb_mbar_arrive(anb_bar + 8u * (anb_s & 1));
+      }}
+      // the last step's words have arrived everywhere before any CTA leaves
+      if (nsteps > 0) anb_mbar_wait(anb_bar + 8u * ((nsteps - 1) & 1), ((nsteps - 1) >> 1) & 1, {err});
+      {nl.join(store)}
+    }}
+    __syncwarp();
+    anb_cluster_sync();
+    if (anb_rank == 0 && threadIdx.x == 0) *{gen.ptr('t')} = t0 + nsteps;
+}}
+"""
+        return Module(gen.assemble([src]), gen.options(), "cluster",
+                      local=("anb_cluster_run", C, block, lay["smem"], C), kernels=["anb_cluster_run"])
+
+    def _update(self, gen, pop, smem, lay) -> str:
+        k, d = pop.id, lay["pop"][pop.id]
+        send = "" if lay["C"] == 1 else f"""
+          if (anb_lane != (int)anb_rank && anb_lane < {lay['C']})
+            anb_st_async(anb_peer + anb_off, anb_m, anb_peer + 8u * (anb_s & 1));"""
+        rec = ""
+        for m in self.net.monitors:
+            if m.population is pop and "spike" in m.variables:
+                ml = self.c.mon_layout[m.id]
+                rec += f"""
+          if (anb_lane == 31 && anb_mon_on{m.id}) {{
+            const int anb_slot = anb_slot0{m.id} + anb_s;
+            if (anb_slot >= 0 && anb_slot < {ml['cap_spike']})
+              {gen.ptr(f'mon{m.id}__spk')}[(unsigned)anb_slot * {ml['words']}u + ((unsigned)(anb_base + anb_q) >> 5)] = anb_m;
+            else
+              anb_report({gen.ptr('err')}, ANB_DEVERR_MONITOR_OVERFLOW);
+          }}"""
+        hook = f"""
+      {{
+        const anb_u32 anb_m = __ballot_sync(0xffffffffu, anb_spiked);
+        if (anb_q - anb_lane < anb_cnt) {{
+          const unsigned anb_off = ((anb_s & 1) ? {d['rep'][1]}u : {d['rep'][0]}u) + 4u * (unsigned)((anb_base + anb_q) >> 5);
+          if (anb_lane == (int)anb_rank) *reinterpret_cast<anb_u32*>(anb_smem + anb_off) = anb_m;{send}{rec}
+        }}
+      }}"""
+        code = gen.neuron_update(pop, local_engine=True, smem=smem, cluster={}, ballot_hook=hook)
+        code = re.sub(r"(anb_rg\d+_\w+)\[anb_q\]", r"\1", code)
+        code = code.replace("for (int anb_q0 = 0; anb_q0 < anb_cnt; anb_q0 += blockDim.x) {",
+                            "{ const int anb_q0 = 0;")
+        return code.replace(f"const int anb_base = anb_base{k}, anb_cnt = anb_cnt{k};",
+                            f"const int anb_base = anb_base{k}, anb_cnt = anb_cnt{k}; (void)anb_base;")
