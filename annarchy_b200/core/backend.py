@@ -70,6 +70,8 @@ class CompiledNetwork:
         self._exchange = None
         # projections delivered through per-neuron inboxes (double precision)
         self.inbox: set = set()
+        # control words of the monitors as last written to the device
+        self._mon_words: dict = {}
 
     # --------------------------------------------------------------- helpers
     def _w(self, w: np.ndarray) -> np.ndarray:
@@ -939,11 +941,17 @@ class CompiledNetwork:
         for mon in self.net.monitors:
             first = self._first_record(mon, t)
             starts[mon.id] = first
-            self.native.write(f"mon{mon.id}__t0", np.array([t], dtype=np.int64))
-            self.native.write(f"mon{mon.id}__t0v", np.array([first], dtype=np.int64))
-            self.native.write(f"mon{mon.id}__start", np.array([mon._start_step], dtype=np.int64))
-            self.native.write(f"mon{mon.id}__on", np.array([1 if mon._recording else 0],
-                                                           dtype=np.int32))
+            # (each write waits for its copy: only what changed, of what is used)
+            words = {"start": mon._start_step, "on": 1 if mon._recording else 0}
+            if "spike" in mon.variables:
+                words["t0"] = t
+            if mon.variables != ["spike"]:
+                words["t0v"] = first
+            for name, value in words.items():
+                if self._mon_words.get((mon.id, name)) != value:
+                    self.native.write(f"mon{mon.id}__{name}", np.array(
+                        [value], dtype=np.int32 if name == "on" else np.int64))
+                    self._mon_words[mon.id, name] = value
         return starts
 
     def end_chunk(self, t, n, starts):
@@ -964,9 +972,8 @@ class CompiledNetwork:
         lay = self.mon_layout[mon.id]
         if "spike" in mon.variables:
             # decoded on the device: only the (step, rank) pairs are copied back
-            steps, ranks = nat.monitor_decode(f"mon{mon.id}__spk", n, lay["words"],
-                                              mon.population.size)
-            mon._append_spikes(steps + t, ranks)
+            mon._append_spikes(*nat.monitor_decode(f"mon{mon.id}__spk", n, lay["words"],
+                                                   mon.population.size, t))
         nrec = 0 if first >= t + n else (t + n - 1 - first) // mon.period_steps + 1
         if nrec > 0:
             rec_steps = first + mon.period_steps * np.arange(nrec)

@@ -502,19 +502,12 @@ class Batch:
             if not any(net.monitors[j]._recording for net in self.networks):
                 continue
             tw = self.total_words[k]
-            steps, bits = self.native.monitor_decode(f"mon{m}__spk", n, tw, tw * 32)
-            woff = self.woff[k]
-            slot = np.searchsorted(woff * 32, bits, side="right") - 1
-            rank = bits - woff[slot] * 32
-            by_slot = np.argsort(slot, kind="stable")
-            bounds = np.searchsorted(slot[by_slot], np.arange(len(self.networks) + 1))
+            steps, ranks, off = self.native.monitor_decode(f"mon{m}__spk", n, tw, tw * 32, t,
+                                                           slots=np.append(self.woff[k], tw))
             for s in range(len(self.networks)):
-                i = int(self.order[s])
-                mon = self.networks[i].monitors[j]
-                if not mon._recording:
-                    continue
-                sel = by_slot[bounds[s]:bounds[s + 1]]
-                mon._append_spikes(steps[sel].astype(np.int64) + t, rank[sel].astype(np.int64))
+                mon = self.networks[int(self.order[s])].monitors[j]
+                if mon._recording:
+                    mon._append_spikes(steps[off[s]:off[s + 1]], ranks[off[s]:off[s + 1]])
 
     def reset(self):
         """Every instance back to the state it was compiled with (attributes

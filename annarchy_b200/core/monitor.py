@@ -197,6 +197,8 @@ class Monitor:
         """(steps, ranks) of all recorded spikes, sorted by step then rank."""
         if not self._spike_steps:
             return np.zeros(0, np.int64), np.zeros(0, np.int64)
+        if len(self._spike_steps) == 1:       # one chunk: sorted as it came
+            return self._spike_steps[0].copy(), self._spike_ranks[0].copy()
         s = np.concatenate(self._spike_steps)
         r = np.concatenate(self._spike_ranks)
         # chunks arrive in time order, each sorted by (step, rank)

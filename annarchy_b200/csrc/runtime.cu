@@ -22,6 +22,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 #include <algorithm>
@@ -167,6 +168,14 @@ struct anb_net {
   int64_t dec_rows_cap = 0;
   int* dec_out = nullptr;
   int64_t dec_out_cap = 0;
+  int64_t dec_last = 0;             // spikes of the last decoding
+  int64_t dec_guess = 4096;         // pairs copied along with the next one's counts
+  int64_t dec_ready = 0;            // of these, in the stage's second half
+  long long* dec_first = nullptr;   // first word of every slot
+  int64_t dec_first_cap = 0;
+  // pinned staging for device-to-host copies, two halves of kStage bytes
+  unsigned char* stage = nullptr;
+  cudaEvent_t stage_ev[2] = {nullptr, nullptr};
   // stop conditions of populations (anb_run_until): the kernel of population
   // `pop` writes the device step into stop_flags[pop] when a neuron satisfies
   // the condition ("any") or when one fails it ("all")
@@ -431,6 +440,69 @@ int build_graph(anb_net* net) {
   return ANB_OK;
 }
 
+constexpr size_t kStage = 1 << 20;
+
+// Pinned stages (2 * kStage bytes) of destroyed networks, for the next ones:
+// allocating one takes about 3 ms. At most kSparePins are kept.
+constexpr size_t kSparePins = 8;
+std::mutex g_pin_mutex;
+std::vector<unsigned char*> g_pins;
+
+int take_stage(anb_net* net) {
+  for (auto& ev : net->stage_ev)
+    if (!ev) ANB_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  {
+    std::lock_guard<std::mutex> lock(g_pin_mutex);
+    if (!g_pins.empty()) {
+      net->stage = g_pins.back();
+      g_pins.pop_back();
+      return ANB_OK;
+    }
+  }
+  void* p = nullptr;
+  ANB_CUDA(cudaHostAlloc(&p, 2 * kStage, cudaHostAllocPortable));
+  net->stage = (unsigned char*)p;
+  return ANB_OK;
+}
+
+// (the network's stream has finished)
+void give_stage(anb_net* net) {
+  if (!net->stage) return;
+  unsigned char* p = net->stage;
+  net->stage = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(g_pin_mutex);
+    if (g_pins.size() < kSparePins) {
+      g_pins.push_back(p);
+      return;
+    }
+  }
+  cudaFreeHost(p);
+}
+
+// Device memory to the host after the stream's work, through the pinned
+// stage: the copy of the next part runs while this one is moved to dst (a
+// copy into pageable memory is staged by the driver in the same way, with two
+// more synchronisations: 32 KB took 21 us and take 14).
+int read_staged(anb_net* net, const void* src, void* dst, size_t bytes) {
+  const size_t parts = (bytes + kStage - 1) / kStage;
+  if (parts > 1) net->dec_ready = 0;   // decoded pairs kept in the second half
+  auto issue = [&](size_t i) -> cudaError_t {
+    const size_t off = i * kStage, n = bytes - off < kStage ? bytes - off : kStage;
+    cudaError_t e = cudaMemcpyAsync(net->stage + (i & 1) * kStage, (const unsigned char*)src + off, n,
+                                    cudaMemcpyDeviceToHost, net->stream);
+    return e != cudaSuccess ? e : cudaEventRecord(net->stage_ev[i & 1], net->stream);
+  };
+  ANB_CUDA(issue(0));
+  for (size_t i = 0; i < parts; ++i) {
+    if (i + 1 < parts) ANB_CUDA(issue(i + 1));
+    ANB_CUDA(cudaEventSynchronize(net->stage_ev[i & 1]));
+    const size_t off = i * kStage, n = bytes - off < kStage ? bytes - off : kStage;
+    std::memcpy((unsigned char*)dst + off, net->stage + (i & 1) * kStage, n);
+  }
+  return ANB_OK;
+}
+
 int write_time(anb_net* net) {
   Array* a = find(net, "t");
   if (!a) return fail(ANB_ERR_STATE, "time counter missing");
@@ -503,10 +575,14 @@ int anb_create(int device, anb_net** out) {
   if (!load_driver()) return fail(ANB_ERR_CUDA, "CUDA driver entry points are unavailable");
   ANB_CUDA(cudaStreamCreateWithFlags(&net->own_stream, cudaStreamNonBlocking));
   net->stream = net->own_stream;
-  int rc = create_array(net.get(), "t", sizeof(long long));
+  int rc = take_stage(net.get());
+  if (rc == ANB_OK) rc = create_array(net.get(), "t", sizeof(long long));
   if (rc == ANB_OK) rc = create_array(net.get(), "dt", sizeof(double));
   if (rc == ANB_OK) rc = create_array(net.get(), "err", 4 * sizeof(int));
-  if (rc != ANB_OK) return rc;
+  if (rc != ANB_OK) {
+    give_stage(net.get());
+    return rc;
+  }
   *out = net.release();
   return ANB_OK;
 }
@@ -526,6 +602,10 @@ int anb_destroy(anb_net* net) {
   if (net->flush_buf) cudaFree(net->flush_buf);
   if (net->dec_rows) cudaFree(net->dec_rows);
   if (net->dec_out) cudaFree(net->dec_out);
+  if (net->dec_first) cudaFree(net->dec_first);
+  give_stage(net);
+  for (auto ev : net->stage_ev)
+    if (ev) cudaEventDestroy(ev);
   if (net->module) g_drv.moduleUnload(net->module);
   for (auto& kv : net->arrays) cudaFree(kv.second.ptr);
   if (net->own_stream) cudaStreamDestroy(net->own_stream);
@@ -620,9 +700,7 @@ int anb_array_read(anb_net* net, const char* name, size_t offset, void* dst, siz
   if (!bytes) return ANB_OK;
   int rc = ensure_device(net);
   if (rc) return rc;
-  ANB_CUDA(cudaMemcpyAsync(dst, (const char*)a->ptr + offset, bytes, cudaMemcpyDeviceToHost, net->stream));
-  ANB_CUDA(cudaStreamSynchronize(net->stream));
-  return ANB_OK;
+  return read_staged(net, (const char*)a->ptr + offset, dst, bytes);
 }
 
 int anb_array_fill_zero(anb_net* net, const char* name) {
@@ -892,7 +970,10 @@ int anb_nvrtc_compile(const char* source, const char* options, char* log, size_t
 }
 
 namespace {
-// Spike-ring decoding on the device: one warp per row.
+// Spike-ring decoding on the device. The ring's words are cut into slots
+// [first[i], first[i + 1]) (one, or one per instance of a batch); row r =
+// slot * steps + step, one warp per row, so the pairs come out by slot, step
+// and rank.
 __device__ __forceinline__ unsigned anb_dec_word(const uint32_t* row, int64_t w, int64_t n) {
   const int64_t valid = n - 32 * w;                 // bits of this word that are neurons
   unsigned m = row[w];
@@ -902,13 +983,16 @@ __device__ __forceinline__ unsigned anb_dec_word(const uint32_t* row, int64_t w,
 }
 
 __global__ void anb_dec_count(const uint32_t* __restrict__ ring, int64_t steps, int64_t words,
-                              int64_t n, long long* __restrict__ counts) {
+                              int64_t n, int64_t rows, const long long* __restrict__ first,
+                              long long* __restrict__ counts) {
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < steps; r += nw) {
-    const uint32_t* row = ring + r * words;
+  for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += nw) {
+    const int64_t slot = r / steps;
+    const uint32_t* row = ring + (r - slot * steps) * words;
+    const int64_t w1 = first[slot + 1];
     int c = 0;
-    for (int64_t w = lane; w < words; w += 32) c += __popc(anb_dec_word(row, w, n));
+    for (int64_t w = first[slot] + lane; w < w1; w += 32) c += __popc(anb_dec_word(row, w, n));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
     if (lane == 0) counts[r] = c;
@@ -953,18 +1037,21 @@ __global__ void anb_dec_scan(long long* __restrict__ counts, int64_t steps) {
   if (threadIdx.x == 0) counts[steps] = carry;
 }
 
-// Pairs in order: out[2k] = step, out[2k+1] = rank.
+// Pairs in order: out[2k] = step, out[2k+1] = rank within the slot.
 __global__ void anb_dec_emit(const uint32_t* __restrict__ ring, int64_t steps, int64_t words,
-                             int64_t n, const long long* __restrict__ offsets, int* __restrict__ out,
+                             int64_t n, int64_t rows, const long long* __restrict__ first,
+                             const long long* __restrict__ offsets, int* __restrict__ out,
                              int64_t capacity) {
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < steps; r += nw) {
-    const uint32_t* row = ring + r * words;
+  for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += nw) {
+    const int64_t slot = r / steps, step = r - slot * steps;
+    const uint32_t* row = ring + step * words;
+    const int64_t wb = first[slot], we = first[slot + 1];
     int64_t base = offsets[r];
-    for (int64_t w0 = 0; w0 < words; w0 += 32) {
+    for (int64_t w0 = wb; w0 < we; w0 += 32) {
       const int64_t w = w0 + lane;
-      unsigned m = w < words ? anb_dec_word(row, w, n) : 0u;
+      unsigned m = w < we ? anb_dec_word(row, w, n) : 0u;
       const int c = __popc(m);
       int incl = c;
 #pragma unroll
@@ -977,8 +1064,8 @@ __global__ void anb_dec_emit(const uint32_t* __restrict__ ring, int64_t steps, i
         const int b = __ffs(m) - 1;
         m &= m - 1;
         if (k < capacity) {
-          out[2 * k] = (int)r;
-          out[2 * k + 1] = (int)(w * 32 + b);
+          out[2 * k] = (int)step;
+          out[2 * k + 1] = (int)((w - wb) * 32 + b);
         }
         ++k;
       }
@@ -988,59 +1075,130 @@ __global__ void anb_dec_emit(const uint32_t* __restrict__ ring, int64_t steps, i
 }
 }  // namespace
 
-int anb_monitor_decode(anb_net* net, const char* array, int64_t steps, int64_t words_per_step,
-                       int64_t n, int32_t* out_steps, int32_t* out_ranks, int64_t capacity,
-                       int64_t* count) {
-  if (!net || !array || !count || steps < 0 || words_per_step < 0 || capacity < 0)
+int anb_monitor_decode_slots(anb_net* net, const char* array, int64_t steps, int64_t words_per_step,
+                             int64_t n, int64_t n_slots, const int64_t* first_word, int64_t* offsets) {
+  if (!net || !array || !offsets || !first_word || steps < 0 || words_per_step < 0 || n_slots < 1)
     return fail(ANB_ERR_ARG, "bad argument");
-  if (capacity > 0 && (!out_steps || !out_ranks)) return fail(ANB_ERR_ARG, "output is NULL");
   Array* a = find(net, array);
   if (!a) return fail(ANB_ERR_ARG, std::string("unknown array ") + array);
   if ((size_t)(steps * words_per_step) * 4 > a->bytes)
     return fail(ANB_ERR_ARG, "more rows requested than the array holds");
   if (steps >= ((int64_t)1 << 31) || words_per_step * 32 >= ((int64_t)1 << 31))
     return fail(ANB_ERR_ARG, "ring too large for 32-bit steps and ranks");
+  for (int64_t i = 0; i < n_slots; ++i)
+    if (first_word[i] < 0 || first_word[i + 1] < first_word[i] || first_word[i + 1] > words_per_step)
+      return fail(ANB_ERR_ARG, "slots must be ascending ranges of the ring's words");
   int rc = ensure_device(net);
   if (rc) return rc;
-  *count = 0;
+  net->dec_last = net->dec_ready = 0;
+  for (int64_t i = 0; i <= n_slots; ++i) offsets[i] = 0;
   if (steps == 0) return ANB_OK;
-  if (net->dec_rows_cap < steps + 1) {
+  const int64_t rows = steps * n_slots;
+  if (net->dec_rows_cap < rows + 1) {
     if (net->dec_rows) cudaFree(net->dec_rows);
     net->dec_rows = nullptr;
     net->dec_rows_cap = 0;
-    ANB_CUDA(cudaMalloc(&net->dec_rows, (size_t)(steps + 1) * sizeof(long long)));
-    net->dec_rows_cap = steps + 1;
+    ANB_CUDA(cudaMalloc(&net->dec_rows, (size_t)(rows + 1) * sizeof(long long)));
+    net->dec_rows_cap = rows + 1;
+  }
+  if (net->dec_first_cap < n_slots + 1) {
+    if (net->dec_first) cudaFree(net->dec_first);
+    net->dec_first = nullptr;
+    net->dec_first_cap = 0;
+    ANB_CUDA(cudaMalloc(&net->dec_first, (size_t)(n_slots + 1) * sizeof(long long)));
+    net->dec_first_cap = n_slots + 1;
+  }
+  ANB_CUDA(cudaMemcpyAsync(net->dec_first, first_word, (size_t)(n_slots + 1) * sizeof(long long),
+                           cudaMemcpyHostToDevice, net->stream));
+  // few spikes are decoded and copied with one wait: pairs up to dec_guess
+  // come along with the counts (a first buffer of 64 KB: larger allocations
+  // take milliseconds)
+  const int64_t stage_pairs = (int64_t)(kStage / (2 * sizeof(int)));
+  if (!net->dec_out) {
+    net->dec_out_cap = 0;
+    ANB_CUDA(cudaMalloc(&net->dec_out, 8192 * 2 * sizeof(int)));
+    net->dec_out_cap = 8192;
   }
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, net->device);
   const uint32_t* ring = static_cast<const uint32_t*>(a->ptr);
-  anb_dec_count<<<sms * 4, 256, 0, net->stream>>>(ring, steps, words_per_step, n, net->dec_rows);
-  anb_dec_scan<<<1, 1024, 0, net->stream>>>(net->dec_rows, steps);
+  const long long* first = net->dec_first;
+  anb_dec_count<<<sms * 4, 256, 0, net->stream>>>(ring, steps, words_per_step, n, rows, first, net->dec_rows);
+  anb_dec_scan<<<1, 1024, 0, net->stream>>>(net->dec_rows, rows);
+  anb_dec_emit<<<sms * 4, 256, 0, net->stream>>>(ring, steps, words_per_step, n, rows, first, net->dec_rows,
+                                                 net->dec_out, net->dec_out_cap);
   ANB_CUDA(cudaGetLastError());
-  long long total = 0;
-  ANB_CUDA(cudaMemcpyAsync(&total, net->dec_rows + steps, sizeof(long long), cudaMemcpyDeviceToHost,
-                           net->stream));
+  // the counts before every slot's first row, and the total
+  const size_t off_bytes = (size_t)(n_slots + 1) * 8;
+  void* off_dst = off_bytes <= kStage ? (void*)net->stage : (void*)offsets;
+  ANB_CUDA(cudaMemcpy2DAsync(off_dst, 8, net->dec_rows, (size_t)steps * 8, 8, (size_t)n_slots + 1,
+                             cudaMemcpyDeviceToHost, net->stream));
+  const int64_t guess = std::min(std::min(stage_pairs, net->dec_out_cap), net->dec_guess);
+  if (guess > 0)
+    ANB_CUDA(cudaMemcpyAsync(net->stage + kStage, net->dec_out, (size_t)guess * 2 * sizeof(int),
+                             cudaMemcpyDeviceToHost, net->stream));
   ANB_CUDA(cudaStreamSynchronize(net->stream));
-  *count = total;
-  const int64_t k = total < capacity ? total : capacity;
-  if (k == 0) return ANB_OK;
-  if (net->dec_out_cap < k) {
-    if (net->dec_out) cudaFree(net->dec_out);
+  if (off_dst != (void*)offsets) std::memcpy(offsets, off_dst, off_bytes);
+  const int64_t total = offsets[n_slots];
+  net->dec_last = total;
+  net->dec_ready = std::min(guess, total);
+  net->dec_guess = total + total / 4 + 512;
+  if (total > net->dec_out_cap) {
+    // more than fitted: emit them again into a larger buffer
+    cudaFree(net->dec_out);
     net->dec_out = nullptr;
     net->dec_out_cap = 0;
-    ANB_CUDA(cudaMalloc(&net->dec_out, (size_t)k * 2 * sizeof(int)));
-    net->dec_out_cap = k;
+    const int64_t cap = total + total / 4;
+    ANB_CUDA(cudaMalloc(&net->dec_out, (size_t)cap * 2 * sizeof(int)));
+    net->dec_out_cap = cap;
+    anb_dec_emit<<<sms * 4, 256, 0, net->stream>>>(ring, steps, words_per_step, n, rows, first,
+                                                   net->dec_rows, net->dec_out, net->dec_out_cap);
+    ANB_CUDA(cudaGetLastError());
   }
-  anb_dec_emit<<<sms * 4, 256, 0, net->stream>>>(ring, steps, words_per_step, n, net->dec_rows,
-                                                 net->dec_out, k);
-  ANB_CUDA(cudaGetLastError());
-  std::vector<int> pairs((size_t)k * 2);
-  ANB_CUDA(cudaMemcpyAsync(pairs.data(), net->dec_out, (size_t)k * 2 * sizeof(int),
-                           cudaMemcpyDeviceToHost, net->stream));
-  ANB_CUDA(cudaStreamSynchronize(net->stream));
+  return ANB_OK;
+}
+
+int anb_monitor_fetch(anb_net* net, int64_t first_step, int64_t* out_steps, int64_t* out_ranks,
+                      int64_t count) {
+  if (!net || count < 0 || (count > 0 && (!out_steps || !out_ranks)))
+    return fail(ANB_ERR_ARG, "bad argument");
+  if (count > net->dec_last) return fail(ANB_ERR_ARG, "more spikes requested than were decoded");
+  int rc = ensure_device(net);
+  if (rc) return rc;
+  const int* p = reinterpret_cast<const int*>(net->stage + kStage);
+  std::vector<int> rest;
+  if (count > net->dec_ready) {
+    rest.resize((size_t)count * 2);
+    rc = read_staged(net, net->dec_out, rest.data(), (size_t)count * 2 * sizeof(int));
+    if (rc) return rc;
+    p = rest.data();
+  }
+  for (int64_t i = 0; i < count; ++i) {
+    out_steps[i] = first_step + p[2 * i];
+    out_ranks[i] = p[2 * i + 1];
+  }
+  net->dec_last = net->dec_ready = 0;
+  return ANB_OK;
+}
+
+int anb_monitor_decode(anb_net* net, const char* array, int64_t steps, int64_t words_per_step,
+                       int64_t n, int32_t* out_steps, int32_t* out_ranks, int64_t capacity,
+                       int64_t* count) {
+  if (!net || !array || !count || capacity < 0) return fail(ANB_ERR_ARG, "bad argument");
+  if (capacity > 0 && (!out_steps || !out_ranks)) return fail(ANB_ERR_ARG, "output is NULL");
+  const int64_t first[2] = {0, words_per_step};
+  int64_t off[2] = {0, 0};
+  *count = 0;
+  int rc = anb_monitor_decode_slots(net, array, steps, words_per_step, n, 1, first, off);
+  if (rc) return rc;
+  *count = off[1];
+  const int64_t k = off[1] < capacity ? off[1] : capacity;
+  std::vector<int64_t> s((size_t)k), r((size_t)k);
+  rc = anb_monitor_fetch(net, 0, s.data(), r.data(), k);
+  if (rc) return rc;
   for (int64_t i = 0; i < k; ++i) {
-    out_steps[i] = pairs[2 * i];
-    out_ranks[i] = pairs[2 * i + 1];
+    out_steps[i] = (int32_t)s[i];
+    out_ranks[i] = (int32_t)r[i];
   }
   return ANB_OK;
 }
@@ -1400,14 +1558,13 @@ int anb_synchronize(anb_net* net) {
   if (!net) return fail(ANB_ERR_ARG, "net is NULL");
   int rc = ensure_device(net);
   if (rc) return rc;
-  ANB_CUDA(cudaStreamSynchronize(net->stream));
+  int code = 0;
+  rc = anb_device_error(net, &code);   // waits for the stream
+  if (rc) return rc;
   if (net->timing) {
     rc = collect_times(net);
     if (rc) return rc;
   }
-  int code = 0;
-  rc = anb_device_error(net, &code);
-  if (rc) return rc;
   switch (code) {
     case 0:
       return ANB_OK;
@@ -1427,8 +1584,8 @@ int anb_device_error(anb_net* net, int* code) {
   if (!net || !code) return fail(ANB_ERR_ARG, "NULL argument");
   Array* a = find(net, "err");
   int v[4] = {0, 0, 0, 0};
-  ANB_CUDA(cudaMemcpyAsync(v, a->ptr, sizeof(v), cudaMemcpyDeviceToHost, net->stream));
-  ANB_CUDA(cudaStreamSynchronize(net->stream));
+  int rc = read_staged(net, a->ptr, v, sizeof(v));
+  if (rc) return rc;
   *code = v[0];
   return ANB_OK;
 }

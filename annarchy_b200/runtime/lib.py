@@ -70,6 +70,9 @@ SIGNATURES = {
                                   C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]),
     "anb_bsr_spmm_simt": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p,
                                     C.c_int, C.c_void_p, C.c_int, C.c_void_p]),
+    "anb_monitor_decode_slots": (C.c_int, [C.c_void_p, C.c_char_p, C.c_int64, C.c_int64, C.c_int64,
+                                           C.c_int64, C.c_void_p, C.c_void_p]),
+    "anb_monitor_fetch": (C.c_int, [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_int64]),
     "anb_monitor_decode": (C.c_int, [C.c_void_p, C.c_char_p, C.c_int64, C.c_int64, C.c_int64,
                                      C.c_void_p, C.c_void_p, C.c_int64, C.POINTER(C.c_int64)]),
     "anb_bank_interleave": (C.c_int, [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p]),
@@ -296,21 +299,22 @@ class NativeNet:
         check("anb_get_stream", self.lib.anb_get_stream(self.h, C.byref(out)))
         return out.value or 0
 
-    def monitor_decode(self, name: str, steps: int, words: int, n: int):
+    def monitor_decode(self, name: str, steps: int, words: int, n: int, t0: int = 0, slots=None):
         """(step, rank) int64 arrays of the spikes in the first `steps` rows of
-        the spike ring `name`, decoded on the device (sorted by step, rank)."""
-        cap = int(max(1024, steps * words))
-        for _ in range(2):
-            s = np.empty(cap, dtype=np.int32)
-            r = np.empty(cap, dtype=np.int32)
-            k = C.c_int64(0)
-            check("anb_monitor_decode", self.lib.anb_monitor_decode(
-                self.h, name.encode(), int(steps), int(words), int(n),
-                s.ctypes.data_as(C.c_void_p), r.ctypes.data_as(C.c_void_p), cap, C.byref(k)))
-            if k.value <= cap:
-                return s[:k.value].astype(np.int64), r[:k.value].astype(np.int64)
-            cap = int(k.value)
-        raise RuntimeError("monitor_decode: spike count changed between calls")
+        the spike ring `name`, decoded on the device (sorted by step, rank),
+        t0 added to the steps. With `slots` (ascending first words, one more
+        than there are slots): sorted by slot, step and rank within the slot,
+        and the slots' offsets as a third array."""
+        first = np.array([0, words] if slots is None else slots, dtype=np.int64)
+        off = np.empty(first.size, dtype=np.int64)
+        check("anb_monitor_decode_slots", self.lib.anb_monitor_decode_slots(
+            self.h, name.encode(), int(steps), int(words), int(n), first.size - 1,
+            first.ctypes.data_as(C.c_void_p), off.ctypes.data_as(C.c_void_p)))
+        k = int(off[-1])
+        s, r = np.empty(k, dtype=np.int64), np.empty(k, dtype=np.int64)
+        check("anb_monitor_fetch", self.lib.anb_monitor_fetch(
+            self.h, int(t0), s.ctypes.data_as(C.c_void_p), r.ctypes.data_as(C.c_void_p), k))
+        return (s, r) if slots is None else (s, r, off)
 
     def zero(self, name: str):
         check("anb_array_fill_zero", self.lib.anb_array_fill_zero(self.h, name.encode()))

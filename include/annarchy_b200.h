@@ -324,6 +324,18 @@ int anb_monitor_decode(anb_net* net, const char* array, int64_t steps, int64_t w
                        int64_t n, int32_t* out_steps, int32_t* out_ranks, int64_t capacity,
                        int64_t* count);
 
+/* The same for a ring whose words are cut into n_slots ranges
+ * [first_word[i], first_word[i+1]) (the instances of a batch): decodes the
+ * spikes by slot, step and rank (ranks count from the slot's first word) and
+ * writes where every slot's begin into offsets[0..n_slots] (the last one is
+ * their number). anb_monitor_fetch then copies the first `count` of them,
+ * first_step added to the steps; a decoding is fetched once. No counterpart
+ * in the reference, whose copies of a network are processes. */
+int anb_monitor_decode_slots(anb_net* net, const char* array, int64_t steps, int64_t words_per_step,
+                             int64_t n, int64_t n_slots, const int64_t* first_word, int64_t* offsets);
+int anb_monitor_fetch(anb_net* net, int64_t first_step, int64_t* out_steps, int64_t* out_ranks,
+                      int64_t count);
+
 int64_t anb_bitmap_decode(const uint32_t* words, int64_t steps, int64_t words_per_step,
                           int64_t n, int64_t* out_steps, int64_t* out_ranks, int64_t capacity);
 
