@@ -70,6 +70,9 @@ class CompiledNetwork:
         self._exchange = None
         # projections delivered through per-neuron inboxes (double precision)
         self.inbox: set = set()
+        # rate tiles of a RateBatch: population -> (first block column, neurons
+        # per copy, copies)
+        self.tc: dict = {}
         # control words of the monitors as last written to the device
         self._mon_words: dict = {}
 
@@ -131,6 +134,7 @@ class CompiledNetwork:
         resident = self._resident_layout()
         for pop in net.populations:
             self._create_population(pop)
+        self._batched_tiles()
         for proj in net.projections:
             self._create_projection(proj)
         for mon in net.monitors:
@@ -169,6 +173,8 @@ class CompiledNetwork:
             nat.set_local_kernel(*mod.local)
         else:
             nat.plan(mod.plan)
+            for pop_id, (first, size1, copies) in self.tc.items():
+                nat.plan_pack(f"pop{pop_id}__r", "tc__xt", copies, size1, first)
             nat.set_graph_steps(int(net._config.get("graph_steps", 32)))
             nat.set_pdl(bool(net._config.get("pdl", True)))
             for pop_id, kernel, grid, block, mode_all in mod.stops:
@@ -673,26 +679,58 @@ class CompiledNetwork:
         name = f"proj{proj.id}__dly" if proj._delay_steps is not None else f"proj{proj.id}__delay"
         self.native.write(name, np.asarray(steps, dtype=np.int32))
 
+    def _batched_tiles(self):
+        """One array of rate tiles for the copies of a RateBatch: every
+        pre-synaptic population's from its first block column on."""
+        projs = [p for p in self.net.projections if getattr(p, "_batched", None) is not None]
+        first = 0
+        for proj in projs:
+            if proj.pre_pop.id not in self.tc:
+                batch, w = proj._batched
+                self.tc[proj.pre_pop.id] = (first, w.shape[1], batch)
+                first += -(-w.shape[1] // 64)
+        if projs:
+            self.native.create_empty("tc__xt", np.uint16, (first * projs[0]._batched[0] * 64,))
+
     def _create_batched_tc(self, proj):
-        """A projection shared by the copies of a RateBatch: the per-copy
-        weights as 64 x 64 bfloat16 blocks in the layout of the tensor-core
-        product (one set for all copies), and the packed-rate scratch."""
+        """The projections of one target shared by the copies of a RateBatch:
+        the per-copy weights as 64 x 64 bfloat16 blocks in the layout of the
+        tensor-core product (one set for all copies), under the first one's
+        name: block row by block row, the blocks of every projection as one
+        run (summed on its own, as by a product per projection)."""
         from ..spmm import TILE, canonical_tiles
         from ..generator.formats import bsr_arrays
         nat = self.native
         k = proj.id
         batch, w = proj._batched
         n_post, n_pre = w.shape
-        d = bsr_arrays(np.arange(n_post), w.indptr, w.indices, w.data, n_pre, TILE)
-        vals = d["values"].reshape(-1, TILE, TILE).transpose(0, 2, 1)      # [block][row][k]
-        n_bcols = -(-n_pre // TILE)
-        nat.create(f"proj{k}__brow", d["block_row_ptr"].astype(np.int32))
-        nat.create(f"proj{k}__bcol", d["block_col"].astype(np.int32))
-        nat.create(f"proj{k}__tiles", to_bf16(canonical_tiles(vals)))
-        nat.create_empty(f"proj{k}__xt", np.uint16, (n_bcols * batch * TILE,))
-        self.layout[k] = {"format": "bsr_tc", "rows": n_post, "nnz": int(w.nnz),
-                          "n_block_rows": int(d["n_block_rows"]), "n_blocks": int(d["n_blocks"]),
-                          "batch": batch, "n_pre": n_pre, "n_post": n_post}
+        group = [p for p in self.net.projections if getattr(p, "_batched", None) is not None
+                 and p.post_pop is proj.post_pop and p.target == proj.target]
+        lay = {"format": "bsr_tc", "rows": n_post, "nnz": int(w.nnz), "batch": batch, "n_pre": n_pre,
+               "n_post": n_post, "merged": proj is not group[0]}
+        self.layout[k] = lay
+        if lay["merged"]:
+            return
+        rows, cols, tiles = [], [], []
+        for p in group:
+            m = p._batched[1]
+            d = bsr_arrays(np.arange(n_post), m.indptr, m.indices, m.data, m.shape[1], TILE)
+            vals = d["values"].reshape(-1, TILE, TILE).transpose(0, 2, 1)      # [block][row][k]
+            tiles.append(to_bf16(canonical_tiles(vals)).reshape(-1, TILE * TILE))
+            rows.append(np.repeat(np.arange(d["n_block_rows"]), np.diff(d["block_row_ptr"])) * len(group)
+                        + len(rows))
+            cols.append(np.asarray(d["block_col"], dtype=np.int64) + self.tc[p.pre_pop.id][0])
+            n_block_rows = int(d["n_block_rows"])
+        rows, cols, tiles = np.concatenate(rows), np.concatenate(cols), np.concatenate(tiles)
+        if len(group) > 1:
+            order = np.argsort(rows, kind="stable")
+            cols, tiles = cols[order], tiles[order]
+        brow = np.zeros(n_block_rows * len(group) + 1, dtype=np.int32)
+        np.cumsum(np.bincount(rows, minlength=brow.size - 1), out=brow[1:])
+        nat.create(f"proj{k}__brow", brow)
+        nat.create(f"proj{k}__bcol", cols.astype(np.int32))
+        nat.create(f"proj{k}__tiles", tiles.reshape(-1))
+        lay.update(n_block_rows=n_block_rows, n_blocks=int(cols.size), parts=len(group))
 
     def _create_projection(self, proj):
         nat = self.native

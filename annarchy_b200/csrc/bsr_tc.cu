@@ -167,15 +167,34 @@ __device__ __forceinline__ void add16_contiguous(float* y, uint32_t taddr, bool 
   }
 }
 
-// Block range of the CTA's i-th block row br (from shared memory when cached).
-__device__ __forceinline__ int2 tc_row(const int2* rows_s, const int* brow_ptr, int i, int br) {
-  return i < kRowCache ? rows_s[i] : make_int2(brow_ptr[br], brow_ptr[br + 1]);
+// Walk of a CTA over its rows: block rows blockIdx.x, blockIdx.x + gridDim.x,
+// ..., each of `parts` runs of blocks (the projections summed into it, every
+// one an accumulation of its own). i: runs so far, sr: the run, q: its part.
+struct TcWalk {
+  int i, sr, q;
+  __device__ __forceinline__ explicit TcWalk(int parts) : i(0), sr(blockIdx.x * parts), q(0) {}
+  __device__ __forceinline__ void next(int parts) {
+    ++i;
+    ++sr;
+    if (++q == parts) {
+      q = 0;
+      sr += (gridDim.x - 1) * parts;
+    }
+  }
+};
+
+// Block range of the CTA's i-th run sr (from shared memory when cached).
+__device__ __forceinline__ int2 tc_row(const int2* rows_s, const int* brow_ptr, int i, int sr) {
+  return i < kRowCache ? rows_s[i] : make_int2(brow_ptr[sr], brow_ptr[sr + 1]);
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+// KEEP: at most one CTA per SM (few block rows), whose epilogue may use the
+// registers; otherwise up to three CTAs share the SM.
+template <bool KEEP>
+__global__ void __launch_bounds__(kThreads, KEEP ? 1 : 3)
 bsr_spmm_tc_kernel(const int* __restrict__ brow_ptr, const int* __restrict__ bcol,
                    const uint16_t* __restrict__ a_tiles, const uint16_t* __restrict__ x_tiles,
-                   int n_block_rows, int batch, float* __restrict__ y, int n_post, int stages,
+                   int n_block_rows, int parts, int batch, float* __restrict__ y, int n_post, int stages,
                    int group, int xmajor, int acc_cols, int tmem_cols, int prefetch, int* err) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2], done;
@@ -211,14 +230,18 @@ bsr_spmm_tc_kernel(const int* __restrict__ brow_ptr, const int* __restrict__ bco
     consumed_n = 0;
     mma_any = 0;
   }
+  const int n_runs = n_block_rows * parts;
   for (int i = threadIdx.x; i < kRowCache; i += kThreads) {
-    const int br = blockIdx.x + i * gridDim.x;
-    if (br < n_block_rows) rows_s[i] = make_int2(brow_ptr[br], brow_ptr[br + 1]);
+    const int sr = (blockIdx.x + (i / parts) * gridDim.x) * parts + i % parts;
+    if (sr < n_runs) rows_s[i] = make_int2(brow_ptr[sr], brow_ptr[sr + 1]);
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = tmem_base;
+  // launched with programmatic dependent launch: everything up to here (the
+  // block rows and barriers, tensor memory) overlaps the previous kernel
+  anb_pdl_enter();
 
   if (warp == 4) {
     // the whole warp: lane i fetches the block column of the stage's i-th
@@ -229,19 +252,28 @@ bsr_spmm_tc_kernel(const int* __restrict__ brow_ptr, const int* __restrict__ bco
     bool ok = true;
     // lane 0 also keeps the weight tiles of the CTA's next `prefetch` blocks
     // on their way into L2 (bulk prefetch), so that their copies into shared
-    // memory wait for L2 rather than HBM: cursor (row i, block range
+    // memory wait for L2 rather than HBM: cursor (run pf, block range
     // [pf_b, pf_e) left in it), blocks prefetched pf_n, blocks copied cp_n
-    int pf_i = 0, pf_br = blockIdx.x, pf_b = 0, pf_e = 0, pf_n = 0, cp_n = 0;
-    if (lane == 0 && prefetch > 0 && pf_br < n_block_rows) {
-      const int2 r0 = tc_row(rows_s, brow_ptr, 0, pf_br);
+    TcWalk pf(parts);
+    int pf_b = 0, pf_e = 0, pf_n = 0, cp_n = 0;
+    if (lane == 0 && prefetch > 0 && pf.sr < n_runs) {
+      const int2 r0 = tc_row(rows_s, brow_ptr, 0, pf.sr);
       pf_b = r0.x;
       pf_e = r0.y;
     }
-    for (int i = 0, br = blockIdx.x; br < n_block_rows && ok; ++i, br += gridDim.x) {
-      const int2 rr = tc_row(rows_s, brow_ptr, i, br);
-      for (int g0 = rr.x; g0 < rr.y; g0 += group) {
+    for (TcWalk at(parts); at.sr < n_runs && ok; at.next(parts)) {
+      const int2 rr = tc_row(rows_s, brow_ptr, at.i, at.sr);
+      int cols = 0;                           // block columns of 32 blocks from c0 on
+      for (int g0 = rr.x, c0 = rr.x; g0 < rr.y; g0 += group) {
         const int gn = rr.y - g0 < group ? rr.y - g0 : group;
-        const int bc = lane < gn ? bcol[g0 + lane] : 0;
+        if (g0 == rr.x || g0 + gn > c0 + 32) {
+          c0 = g0;
+          cols = c0 + lane < rr.y ? bcol[c0 + lane] : 0;
+        }
+        // a thread's bulk copies are served one after another: the stages'
+        // copies are dealt to the lanes in turn
+        const int l0 = KEEP ? k * (group + 1) & 31 : 0, li = (lane - l0 - (KEEP ? 1 : 0)) & 31;
+        const int bc = __shfl_sync(0xffffffffu, cols, (g0 - c0 + li) & 31);
         if (k >= stages) {
           const bool w = __all_sync(0xffffffffu, mbar_wait(&empty[s], ph ^ 1u, &abort_flag));
           if (!w) {
@@ -256,11 +288,11 @@ bsr_spmm_tc_kernel(const int* __restrict__ brow_ptr, const int* __restrict__ bco
         unsigned char* st = smem + s * stage_bytes;
         if (lane == 0) mbar_expect_tx(&full[s], (unsigned)gn * (kTileBytes + x_bytes));
         __syncwarp();
-        if (lane == 0) bulk_load(st, a_tiles + (size_t)g0 * (kTile * kTile), (unsigned)gn * kTileBytes, &full[s]);
-        if (lane < gn) bulk_load(st + x_off + lane * x_bytes, x_tiles + (size_t)bc * batch * kTile, x_bytes, &full[s]);
+        if (lane == l0) bulk_load(st, a_tiles + (size_t)g0 * (kTile * kTile), (unsigned)gn * kTileBytes, &full[s]);
+        if (li < gn) bulk_load(st + x_off + li * x_bytes, x_tiles + (size_t)bc * batch * kTile, x_bytes, &full[s]);
         if (lane == 0 && prefetch > 0) {
           cp_n += gn;
-          while (pf_br < n_block_rows && pf_n < cp_n + prefetch) {
+          while (pf.sr < n_runs && pf_n < cp_n + prefetch) {
             const int want = min(pf_e - pf_b, cp_n + prefetch - pf_n);
             if (want > 0) {
               asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
@@ -269,11 +301,10 @@ bsr_spmm_tc_kernel(const int* __restrict__ brow_ptr, const int* __restrict__ bco
               pf_b += want;
               pf_n += want;
             }
-            if (pf_b >= pf_e) {               // next row of this CTA
-              ++pf_i;
-              pf_br += gridDim.x;
-              if (pf_br < n_block_rows) {
-                const int2 r = tc_row(rows_s, brow_ptr, pf_i, pf_br);
+            if (pf_b >= pf_e) {               // next run of this CTA
+              pf.next(parts);
+              if (pf.sr < n_runs) {
+                const int2 r = tc_row(rows_s, brow_ptr, pf.i, pf.sr);
                 pf_b = r.x;
                 pf_e = r.y;
               }
@@ -309,8 +340,8 @@ bsr_spmm_tc_kernel(const int* __restrict__ brow_ptr, const int* __restrict__ bco
       int s = 0, k = 0, t = 0;                // stage, stages consumed, non-empty rows done
       unsigned ph = 0;
       bool ok = true;
-      for (int i = 0, br = blockIdx.x; br < n_block_rows && ok; ++i, br += gridDim.x) {
-        const int2 rr = tc_row(rows_s, brow_ptr, i, br);
+      for (TcWalk at(parts); at.sr < n_runs && ok; at.next(parts)) {
+        const int2 rr = tc_row(rows_s, brow_ptr, at.i, at.sr);
         if (rr.y == rr.x) continue;
         const int a = t & 1, v = t >> 1;
         if (v > 0 && !mbar_wait(&acc_empty[a], (v - 1) & 1, &abort_flag)) {
@@ -366,8 +397,81 @@ bsr_spmm_tc_kernel(const int* __restrict__ brow_ptr, const int* __restrict__ bco
     // epilogue warps 0-3
     const bool vec = (n_post & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
     int t = 0;
-    for (int i = 0, br = blockIdx.x; br < n_block_rows; ++i, br += gridDim.x) {
-      const int2 rr = tc_row(rows_s, brow_ptr, i, br);
+    // Up to 64 values a thread (one instance's 64 rows, or one row of up to 64
+    // instances) stay in registers over the runs of a block row: read while
+    // the first run's products are under way, written after the last one's.
+    const bool keep = KEEP && (xmajor ? batch == 128 : batch <= 64);
+    bool loaded = false;
+    float sum[KEEP ? 64 : 1];
+    for (TcWalk at(parts); at.sr < n_runs; at.next(parts)) {
+      const int2 rr = tc_row(rows_s, brow_ptr, at.i, at.sr);
+      const int br = at.sr / parts;
+      if constexpr (KEEP) if (keep) {
+        const int r0 = br * kTile, row = r0 + 16 * warp + lane;
+        const int valid = xmajor ? min(kTile, n_post - r0) : 0;
+        const bool mine = xmajor || (lane < 16 && row < n_post);
+        float* yb = xmajor ? y + (size_t)(32 * warp + lane) * n_post + r0 : y + row;
+        const bool whole = vec && valid == kTile;
+        if (rr.y > rr.x) {
+          if (!loaded) {
+            loaded = true;
+            if (whole) {
+#pragma unroll
+              for (int j = 0; j < 64; j += 4) {
+                const float4 o = *reinterpret_cast<const float4*>(yb + j);
+                sum[j] = o.x; sum[j + 1] = o.y; sum[j + 2] = o.z; sum[j + 3] = o.w;
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 64; ++j)
+                sum[j] = xmajor ? (j < valid ? yb[j] : 0.f)
+                                : (mine && j < batch ? yb[(size_t)j * n_post] : 0.f);
+            }
+          }
+          const int a = t & 1, v = t >> 1;
+          const bool ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[a], v & 1, &abort_flag));
+          if (!ok) {
+            if (lane == 0) {
+              anb_report(err, ANB_DEVERR_BARRIER_TIMEOUT);
+              abort_flag = 1;
+            }
+            break;
+          }
+          tc_fence_after();
+          const uint32_t tw = tbase + ((uint32_t)(32 * warp) << 16) + (uint32_t)(a * acc_cols);
+#pragma unroll
+          for (int c0 = 0; c0 < 64; c0 += 16) {
+            if (xmajor || c0 < batch) {
+              uint32_t r[16];
+              tmem_ld16(tw + (uint32_t)c0, r);
+#pragma unroll
+              for (int j = 0; j < 16; ++j) sum[c0 + j] += __uint_as_float(r[j]);
+            }
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_empty[a]);
+          ++t;
+        }
+        if (at.q == parts - 1 && loaded) {
+          loaded = false;
+          if (whole) {
+#pragma unroll
+            for (int j = 0; j < 64; j += 4)
+              *reinterpret_cast<float4*>(yb + j) = make_float4(sum[j], sum[j + 1], sum[j + 2], sum[j + 3]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 64; ++j) {
+              if (xmajor) {
+                if (j < valid) yb[j] = sum[j];
+              } else if (mine && j < batch) {
+                yb[(size_t)j * n_post] = sum[j];
+              }
+            }
+          }
+        }
+        continue;
+      }
       if (rr.y == rr.x) continue;
       const int a = t & 1, v = t >> 1;
       const bool ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[a], v & 1, &abort_flag));
@@ -536,6 +640,14 @@ int g_tc_prefetch = 4;
 
 extern "C" {
 
+// anb_bsr_spmm_tc for the step plan (csrc/runtime.cu): brow_ptr has `parts`
+// runs of blocks per block row, added to y one after another (as one product
+// per run would); with pdl, launched while the stream's previous kernel may
+// still run.
+int anb_bsr_spmm_tc_after(const int* brow_ptr, const int* bcol, const uint16_t* a_tiles,
+                          int n_block_rows, int parts, const uint16_t* x_tiles, int batch, float* y,
+                          int n_post, int* err, void* stream, int pdl);
+
 int anb_bsr_tc_pack_x(const float* x, int batch, int n_pre, uint16_t* x_tiles, void* stream) {
   if (!x || !x_tiles || batch <= 0 || batch % 16 != 0 || batch > 256 || n_pre <= 0) return 2;
   const int n_bcols = (n_pre + kTile - 1) / kTile;
@@ -562,7 +674,14 @@ int anb_bsr_spmm_tc_prefetch(int blocks) {
 int anb_bsr_spmm_tc(const int* brow_ptr, const int* bcol, const uint16_t* a_tiles,
                     int n_block_rows, const uint16_t* x_tiles, int batch, float* y, int n_post,
                     int* err, void* stream) {
-  if (!brow_ptr || !bcol || !a_tiles || !x_tiles || !y || n_block_rows < 0) return 2;
+  return anb_bsr_spmm_tc_after(brow_ptr, bcol, a_tiles, n_block_rows, 1, x_tiles, batch, y, n_post, err,
+                               stream, 0);
+}
+
+int anb_bsr_spmm_tc_after(const int* brow_ptr, const int* bcol, const uint16_t* a_tiles,
+                          int n_block_rows, int parts, const uint16_t* x_tiles, int batch, float* y,
+                          int n_post, int* err, void* stream, int pdl) {
+  if (!brow_ptr || !bcol || !a_tiles || !x_tiles || !y || n_block_rows < 0 || parts < 1) return 2;
   if (batch < 16 || batch > 256 || batch % 16 != 0) return 2;
   if (n_block_rows == 0) return 0;
   static int sm_count = 0;
@@ -599,6 +718,14 @@ int anb_bsr_spmm_tc(const int* brow_ptr, const int* bcol, const uint16_t* a_tile
     stages = (int)((200u << 10) / (group * block_bytes));
     if (stages > 4) stages = 4;
   }
+  if (n_block_rows <= sm_count) {
+    // at most one row per SM: nothing but the row's own stages overlaps its
+    // copies, so the ring is as deep as shared memory allows
+    per_sm = 1;
+    group = 4 * block_bytes <= (104u << 10) ? 2 : 1;
+    stages = (int)((200u << 10) / (group * block_bytes));
+    if (stages > 8) stages = 8;
+  }
   if (g_tc_per_sm > 0) per_sm = g_tc_per_sm;
   if (g_tc_stages > 0) stages = g_tc_stages;
   if (g_tc_group > 0) group = g_tc_group;
@@ -606,14 +733,26 @@ int anb_bsr_spmm_tc(const int* brow_ptr, const int* bcol, const uint16_t* a_tile
   if (stages < 2 || stages > kMaxStages || group < 1 || group > 8 || smem > (200u << 10) ||
       per_sm * tmem_cols > 512)
     return 2;
-  if (cudaFuncSetAttribute(bsr_spmm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
+  // few block rows: one CTA per SM, unless a shape for more was asked for
+  auto kernel = n_block_rows <= sm_count && per_sm == 1 ? bsr_spmm_tc_kernel<true> : bsr_spmm_tc_kernel<false>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return 4;
   const int grid = n_block_rows < per_sm * sm_count ? n_block_rows : per_sm * sm_count;
-  bsr_spmm_tc_kernel<<<grid, kThreads, smem, (cudaStream_t)stream>>>(
-      brow_ptr, bcol, a_tiles, x_tiles, n_block_rows, batch, y, n_post, stages, group, xmajor,
-      acc_cols, tmem_cols, g_tc_prefetch, err);
-  return cudaGetLastError() == cudaSuccess ? 0 : 4;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = (cudaStream_t)stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, brow_ptr, bcol, a_tiles, x_tiles, n_block_rows, parts, batch, y,
+                            n_post, stages, group, xmajor, acc_cols, tmem_cols, g_tc_prefetch,
+                            err) == cudaSuccess
+             ? 0
+             : 4;
 }
 
 int anb_bsr_spmm_simt(const int* brow_ptr, const int* bcol, const uint16_t* a_tiles,

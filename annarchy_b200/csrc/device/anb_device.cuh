@@ -63,6 +63,15 @@ __device__ __forceinline__ double anb_wf(double w) { return w; }
 __device__ __forceinline__ float anb_wf(float w) { return w; }
 __device__ __forceinline__ float anb_wf(anb_bf16 w) { return anb_bf16_to_f32(w); }
 
+// Rate r of neuron k of copy b, rounded to bfloat16 (nearest even), into the
+// 64-neuron tiles of the batched block product: element (b, k % 64) of tile
+// k / 64 in 8 x 8 core matrices of 16-byte rows.
+__device__ __forceinline__ void anb_store_tile(anb_bf16* tiles, int b, int k, int copies, float r) {
+  const anb_u32 u = __float_as_uint(r);
+  tiles[(size_t)(k >> 6) * copies * 64 + ((b >> 3) * 8 + ((k & 63) >> 3)) * 64 + (b & 7) * 8 + (k & 7)] =
+      (anb_bf16)((u + 0x7FFFu + ((u >> 16) & 1u)) >> 16);
+}
+
 // ---- spike bitmaps -------------------------------------------------------------
 __device__ __forceinline__ bool anb_bit(const anb_u32* bits, int i) {
   return (bits[i >> 5] >> (i & 31)) & 1u;

@@ -29,6 +29,10 @@
 
 #include "../../include/annarchy_b200.h"
 
+extern "C" int anb_bsr_spmm_tc_after(const int* brow_ptr, const int* bcol, const uint16_t* a_tiles,
+                                     int n_block_rows, int parts, const uint16_t* x_tiles, int batch,
+                                     float* y, int n_post, int* err, void* stream, int pdl);
+
 namespace {
 
 thread_local std::string g_error;
@@ -106,7 +110,7 @@ struct Array {
 };
 
 // Plan entries that are library operations rather than module kernels.
-enum { kOpKernel = 0, kOpBsrTc = 1 };
+enum { kOpKernel = 0, kOpBsrTc = 1, kOpBsrShared = 2 };
 
 struct Launch {
   std::string name;
@@ -117,7 +121,7 @@ struct Launch {
   bool cooperative = false;  // all CTAs resident at once (grid-wide barriers)
   int op = kOpKernel;
   // kOpBsrTc: arrays block_row_ptr, block_col, tiles, x, x_tiles, y and the
-  // sizes n_block_rows, batch, n_pre, n_post
+  // sizes n_block_rows, batch, n_pre, n_post (kOpBsrShared: no x, the runs per block row for n_pre)
   std::string arr[6];
   int iarg[4] = {0, 0, 0, 0};
 };
@@ -193,6 +197,13 @@ struct anb_net {
     int64_t period = 1;
   };
   std::vector<Record> records;
+  // rates packed into shared bfloat16 tiles at the start of every run; the
+  // step's update kernels keep the tiles up to date
+  struct Pack {
+    std::string x, tiles;
+    int batch = 0, n_pre = 0, first_block = 0;
+  };
+  std::vector<Pack> packs;
 };
 
 namespace {
@@ -257,7 +268,25 @@ int launch_bsr_tc(anb_net* net, const Launch& l, cudaStream_t st) {
   return ANB_OK;
 }
 
+int launch_bsr_shared(anb_net* net, const Launch& l, cudaStream_t st, bool pdl) {
+  void* p[6] = {};
+  for (int i = 0; i < 6; ++i) {
+    if (i == 3) continue;
+    Array* a = find(net, l.arr[i].c_str());
+    if (!a) return fail(ANB_ERR_STATE, l.name + ": array " + l.arr[i] + " is missing");
+    p[i] = a->ptr;
+  }
+  Array* err = find(net, "err");
+  const int rc = anb_bsr_spmm_tc_after((const int*)p[0], (const int*)p[1], (const uint16_t*)p[2], l.iarg[0], l.iarg[2],
+                                       (const uint16_t*)p[4], l.iarg[1], (float*)p[5], l.iarg[3],
+                                       err ? (int*)err->ptr : nullptr, st, pdl ? 1 : 0);
+  if (rc == 2) return fail(ANB_ERR_ARG, l.name + ": the block product rejected its sizes");
+  if (rc != 0) return fail(ANB_ERR_CUDA, l.name + ": block product launch failed");
+  return ANB_OK;
+}
+
 int launch(anb_net* net, const Launch& l, void** params, cudaStream_t on = nullptr, bool pdl = false) {
+  if (l.op == kOpBsrShared) return launch_bsr_shared(net, l, on ? on : net->stream, pdl);
   if (l.op == kOpBsrTc) return launch_bsr_tc(net, l, on ? on : net->stream);
   if (l.cooperative) {
     CUlaunchAttribute attr;
@@ -768,6 +797,7 @@ int anb_module_load(anb_net* net, const char* source, const char* options) {
   ANB_CUDA(cudaStreamSynchronize(net->stream));
   drop_graph(net);
   net->plan.clear();
+  net->packs.clear();
   net->stops.clear();
   net->has_local = false;
   if (net->module) {
@@ -1279,6 +1309,7 @@ int anb_plan_clear(anb_net* net) {
   if (!net) return fail(ANB_ERR_ARG, "net is NULL");
   drop_graph(net);
   net->plan.clear();
+  net->packs.clear();
   return ANB_OK;
 }
 
@@ -1374,6 +1405,56 @@ int anb_plan_add_bsr_tc(anb_net* net, const char* prefix, const char* x_array,
   return ANB_OK;
 }
 
+int anb_plan_add_bsr_shared(anb_net* net, const char* prefix, const char* tiles_array,
+                            const char* y_array, int n_block_rows, int parts, int batch, int n_post) {
+  if (!net || !prefix || !tiles_array || !y_array) return fail(ANB_ERR_ARG, "NULL argument");
+  if (batch < 16 || batch > 256 || batch % 16)
+    return fail(ANB_ERR_ARG, "batch must be a multiple of 16 between 16 and 256");
+  if (n_block_rows < 0 || parts < 1 || n_post <= 0 || n_block_rows * 64 < n_post)
+    return fail(ANB_ERR_ARG, "inconsistent block-sparse sizes");
+  Launch l;
+  const std::string p(prefix);
+  l.name = p + "_bsr_tc";
+  l.op = kOpBsrShared;
+  const std::string names[6] = {p + "__brow", p + "__bcol", p + "__tiles", "", tiles_array, y_array};
+  for (int i = 0; i < 6; ++i) {
+    if (i != 3 && !find(net, names[i].c_str())) return fail(ANB_ERR_ARG, "unknown array " + names[i]);
+    l.arr[i] = names[i];
+  }
+  if (find(net, names[0].c_str())->bytes < 4 * ((size_t)n_block_rows * parts + 1))
+    return fail(ANB_ERR_ARG, names[0] + " holds too few runs of blocks");
+  if (find(net, y_array)->bytes < sizeof(float) * (size_t)batch * n_post)
+    return fail(ANB_ERR_ARG, std::string(y_array) + " holds fewer than batch x n_post floats");
+  l.iarg[0] = n_block_rows;
+  l.iarg[1] = batch;
+  l.iarg[2] = parts;
+  l.iarg[3] = n_post;
+  drop_graph(net);
+  net->plan.push_back(l);
+  return ANB_OK;
+}
+
+int anb_plan_pack(anb_net* net, const char* x_array, const char* tiles_array, int batch, int n_pre,
+                  int first_block) {
+  if (!net || !x_array || !tiles_array) return fail(ANB_ERR_ARG, "NULL argument");
+  if (batch < 16 || batch > 256 || batch % 16 || n_pre <= 0 || first_block < 0)
+    return fail(ANB_ERR_ARG, "inconsistent sizes");
+  Array* x = find(net, x_array);
+  Array* t = find(net, tiles_array);
+  if (!x || !t) return fail(ANB_ERR_ARG, std::string("unknown array ") + (x ? tiles_array : x_array));
+  if (x->bytes < sizeof(float) * (size_t)batch * n_pre ||
+      t->bytes < 2 * ((size_t)first_block + (n_pre + 63) / 64) * batch * 64)
+    return fail(ANB_ERR_ARG, "the arrays are too small for the rates and their tiles");
+  anb_net::Pack p;
+  p.x = x_array;
+  p.tiles = tiles_array;
+  p.batch = batch;
+  p.n_pre = n_pre;
+  p.first_block = first_block;
+  net->packs.push_back(p);
+  return ANB_OK;
+}
+
 int anb_set_local_kernel(anb_net* net, const char* kernel, unsigned grid, unsigned block,
                          unsigned shared_bytes) {
   Launch l;
@@ -1466,6 +1547,15 @@ int anb_run(anb_net* net, int64_t nsteps) {
     }
     net->t += nsteps;
     return ANB_OK;
+  }
+  for (const auto& p : net->packs) {
+    Array* x = find(net, p.x.c_str());
+    Array* tl = find(net, p.tiles.c_str());
+    if (!x || !tl) return fail(ANB_ERR_STATE, p.x + " or " + p.tiles + " is missing");
+    if (anb_bsr_tc_pack_x((const float*)x->ptr, p.batch, p.n_pre,
+                          (uint16_t*)tl->ptr + (size_t)p.first_block * p.batch * 64, net->stream) != 0)
+      return fail(ANB_ERR_CUDA, "packing of " + p.x + " failed");
+    net->pdl_prev = false;
   }
   int64_t remaining = nsteps;
   if (!net->timing && net->graph_steps > 1 && nsteps >= net->graph_steps) {

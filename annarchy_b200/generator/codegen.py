@@ -557,6 +557,13 @@ class CodeGenerator:
             rv = "r" if "r" in names else f"{gsrc('r')}[anb_i]"
             stores.append(f"{self.ptr(f'pop{k}___delayed_r')}[(size_t)anb_ring_slot(t, {self.slots(pop)}) * "
                           f"{self.c.ring_stride(pop)} + anb_i] = {rv};")
+        if grid_path and pop.id in self.c.tc:
+            # this step's rate, rounded to bfloat16 (nearest even), into the tiles
+            # the tensor-core product reads (layout of anb_bsr_tc_pack_x)
+            first, size1, copies = self.c.tc[pop.id]
+            rv = "r" if "r" in names else f"{gsrc('r')}[anb_i]"
+            stores.append(f"anb_store_tile({self.ptr('tc__xt')} + (size_t){first * copies * 64}, anb_i / {size1}, "
+                          f"anb_i % {size1}, {copies}, {rv});")
         ballot = ""
         listed = (spiking and cluster is None and not local_engine and not self.exact
                   and self.c.spike_lists)
@@ -1244,11 +1251,14 @@ extern "C" __global__ void __launch_bounds__({bounds}) {nm}() {{
             return self.custom_psp_kernel(proj), [(name, grid_for(lay["rows"]), BLOCK, 0)]
         if fmt == "bsr_tc":
             # copies of the network sharing the weights: one tensor-core
-            # product for all of them (a library operation of the plan)
-            op = {"prefix": f"proj{k}", "x": f"pop{proj.pre_pop.id}__r",
+            # product for all of them and for all projections of the target (a
+            # library operation of the plan)
+            if lay["merged"]:
+                return "", []
+            op = {"prefix": f"proj{k}", "tiles": "tc__xt",
                   "y": f"pop{proj.post_pop.id}___sum_{proj.target}",
-                  "n_block_rows": lay["n_block_rows"], "batch": lay["batch"],
-                  "n_pre": lay["n_pre"], "n_post": lay["n_post"]}
+                  "n_block_rows": lay["n_block_rows"], "parts": lay["parts"], "batch": lay["batch"],
+                  "n_post": lay["n_post"]}
             return "", [(op, 0, 0, 0)]
         if proj._delay_steps is not None:
             # one delay per synapse: CSR rows read the rate ring per synapse

@@ -109,6 +109,9 @@ SIGNATURES = {
                                                C.POINTER(C.c_longlong)]),
     "anb_set_local_kernel_cooperative": (C.c_int, [C.c_void_p, C.c_char_p, C.c_uint, C.c_uint,
                                                    C.POINTER(C.c_uint)]),
+    "anb_plan_add_bsr_shared": (C.c_int, [C.c_void_p, C.c_char_p, C.c_char_p, C.c_char_p, C.c_int,
+                                          C.c_int, C.c_int, C.c_int]),
+    "anb_plan_pack": (C.c_int, [C.c_void_p, C.c_char_p, C.c_char_p, C.c_int, C.c_int, C.c_int]),
     "anb_plan_add_bsr_tc": (C.c_int, [C.c_void_p, C.c_char_p, C.c_char_p, C.c_char_p, C.c_int,
                                       C.c_int, C.c_int, C.c_int, C.c_int]),
     "anb_set_seed": (C.c_int, [C.c_void_p, C.c_uint64, C.c_int, C.c_int]),
@@ -479,15 +482,18 @@ class NativeNet:
         for entry in launches:
             if isinstance(entry[0], dict):          # a library operation
                 op = entry[0]
-                check("anb_plan_add_bsr_tc", self.lib.anb_plan_add_bsr_tc(
-                    self.h, op["prefix"].encode(), op["x"].encode(), op["y"].encode(),
-                    op["n_block_rows"], op["batch"], op["n_pre"], op["n_post"],
-                    entry[4] if len(entry) > 4 else 0))
+                check("anb_plan_add_bsr_shared", self.lib.anb_plan_add_bsr_shared(
+                    self.h, op["prefix"].encode(), op["tiles"].encode(), op["y"].encode(),
+                    op["n_block_rows"], op["parts"], op["batch"], op["n_post"]))
                 continue
             name, grid, block, smem = entry[:4]
             group = entry[4] if len(entry) > 4 else 0
             check("anb_plan_add_concurrent", self.lib.anb_plan_add_concurrent(
                 self.h, name.encode(), grid, block, smem, group))
+
+    def plan_pack(self, x: str, tiles: str, batch: int, n_pre: int, first_block: int):
+        check("anb_plan_pack", self.lib.anb_plan_pack(self.h, x.encode(), tiles.encode(), batch, n_pre,
+                                                      first_block))
 
     def set_local_kernel(self, name, grid, block, smem, cluster: int = 1):
         if cluster == -1:                       # cooperative: the runtime sizes the grid
@@ -635,6 +641,9 @@ class DryNative:
 
     def load_module(self, source, options):
         self.source, self.options = source, options
+
+    def plan_pack(self, *a):
+        pass
 
     def plan(self, launches):
         self.launches = list(launches)

@@ -400,6 +400,19 @@ int anb_plan_add_bsr_tc(anb_net* net, const char* prefix, const char* x_array,
                         const char* y_array, int n_block_rows, int batch, int n_pre, int n_post,
                         int group);
 
+/* The same with tiles that several products share: "<prefix>__bcol" counts
+ * block columns of tiles_array, which may hold the tiles of several arrays of
+ * rates one after another; "<prefix>__brow" has `parts` runs of blocks per
+ * block row (one per projection of the target), added one after another; and
+ * nothing is packed per step: anb_plan_pack names the arrays packed at the
+ * start of every run (x_array, batch x n_pre, from block first_block on), and
+ * the step's update kernels store the rates they change in the tiles too.
+ * anb_plan_clear forgets both. */
+int anb_plan_add_bsr_shared(anb_net* net, const char* prefix, const char* tiles_array,
+                            const char* y_array, int n_block_rows, int parts, int batch, int n_post);
+int anb_plan_pack(anb_net* net, const char* x_array, const char* tiles_array, int batch, int n_pre,
+                  int first_block);
+
 /* Launch shape of anb_bsr_spmm_tc for this process: resident CTAs per SM
  * (1-4), shared-memory stages per CTA (2-12) and consecutive blocks of a row
  * per stage (1-8); 0 keeps the automatic choice (two stages; two blocks per
