@@ -70,6 +70,8 @@ class CompiledNetwork:
         self._exchange = None
         # projections delivered through per-neuron inboxes (double precision)
         self.inbox: set = set()
+        # the cluster form with per-warp masks, when it runs the network
+        self.masks = None
         # rate tiles of a RateBatch: population -> (first block column, neurons
         # per copy, copies)
         self.tc: dict = {}
@@ -141,6 +143,10 @@ class CompiledNetwork:
             self._create_monitor(mon)
         for pop in net.populations:
             pop._init_state = {k: v.copy() for k, v in pop._host.items()}
+        masks = self._delay_masks()
+        if masks and self._load_masks(masks):
+            self.masks = masks
+            return
         if self.engine == "local":
             self._build_cluster()
             return
@@ -152,6 +158,10 @@ class CompiledNetwork:
             self.write_constants()
             nat.set_local_kernel(*self.module.local)
             return
+        self._build_plan()
+
+    def _build_plan(self):
+        net, nat = self.net, self.native
         gen = CodeGenerator(self)
         if self.engine == "local":
             self._local_layout()
@@ -201,14 +211,21 @@ class CompiledNetwork:
         launches, and 17.4 against 16.1 us on its 200k-neuron version."""
         return bool(self.net._config.get("persistent", False))
 
-    def _build_cluster(self):
-        """Fast spiking engine on one thread-block cluster: the smallest
-        cluster (up to 16 CTAs) whose shared memory holds the state and the
-        synapses; otherwise 8 CTAs with the synapses read from global memory.
-        A cluster the device cannot schedule falls back the same way."""
-        from ..runtime.lib import BackendError
+    def _delay_masks(self):
+        """The Masks of a small spiking network with synaptic delays (the grid
+        engine's form for it: one cluster instead of launches per step), None
+        when the network does not qualify."""
+        if (self.engine != "grid" or self.net._config.get("engine", "auto") != "auto" or self.shard
+                or all(p.max_delay <= 1 for p in self.net.projections)
+                or any(getattr(p, "stop_condition", None) for p in self.net.populations)
+                or self.net._config.get("persistent") or not self._local_possible(delays=True)[0]):
+            return None
         masks = Masks(self)
-        for lay in masks.choose() if masks.possible() else []:
+        return masks if masks.possible() and masks.choose() else None
+
+    def _load_masks(self, masks) -> bool:
+        from ..runtime.lib import BackendError
+        for lay in masks.choose():
             masks.create_arrays(lay)
             mod = masks.module(lay)
             try:
@@ -218,6 +235,39 @@ class CompiledNetwork:
             except BackendError:
                 continue                       # a cluster the device cannot schedule
             self.module = mod
+            return True
+        return False
+
+    def _leave_masks(self):
+        """From the cluster form of a delayed network to the grid engine's
+        plan, which reads the same bitmaps and states: its projections now
+        carry different weights."""
+        nat = self.native
+        self.masks = None
+        self._build_plan()
+        t = nat.get_time()
+        for pop in self.net.populations:
+            name = f"pop{pop.id}__spn"
+            if name not in nat.arrays or t == 0:
+                continue
+            # the last step's spikes as the list that the plan transmits from
+            slot, words = (t - 1) % self.slots[pop.id], (pop.size + 31) // 32
+            last = nat.read(f"pop{pop.id}__spk", count=words, offset=slot * words)
+            ranks = bitmap_to_spikes_numpy(last.reshape(1, -1), pop.size)[1].astype(np.int32)
+            count = np.zeros(2, dtype=np.int32)
+            if nat.read(name).any() and ranks.size:
+                count[(t - 1) & 1] = ranks.size
+                nat.write(f"pop{pop.id}__spl", ranks, offset_bytes=4 * pop.size * ((t - 1) & 1))
+            nat.write(name, count)
+
+    def _build_cluster(self):
+        """Fast spiking engine on one thread-block cluster: the smallest
+        cluster (up to 16 CTAs) whose shared memory holds the state and the
+        synapses; otherwise 8 CTAs with the synapses read from global memory.
+        A cluster the device cannot schedule falls back the same way."""
+        from ..runtime.lib import BackendError
+        masks = Masks(self)
+        if masks.possible() and self._load_masks(masks):
             self.engine = "cluster"
             return
         want = self.net._config.get("cluster_size")
@@ -295,9 +345,9 @@ class CompiledNetwork:
             return "grid"
         return "local" if ok else "grid"
 
-    def _local_possible(self):
+    def _local_possible(self, delays: bool = False):
         net = self.net
-        if any(p.max_delay > 1 for p in net.projections):
+        if not delays and any(p.max_delay > 1 for p in net.projections):
             return False, "synaptic delays"
         if any(p.neuron_type.type != "spike" for p in net.populations):
             return False, "rate-coded populations"
@@ -678,6 +728,8 @@ class CompiledNetwork:
     def write_delays(self, proj, steps: np.ndarray):
         name = f"proj{proj.id}__dly" if proj._delay_steps is not None else f"proj{proj.id}__delay"
         self.native.write(name, np.asarray(steps, dtype=np.int32))
+        if self.masks is not None:
+            self.masks.write_delays(proj)
 
     def _batched_tiles(self):
         """One array of rate tiles for the copies of a RateBatch: every
@@ -1160,6 +1212,8 @@ class CompiledNetwork:
             if name not in proj._host_semi and name not in proj._host_attr:
                 proj._global_values[name] = float(np.asarray(arr).reshape(-1)[0])
             return
+        if name == "w" and self.masks is not None and not self.masks.write_weights(proj):
+            self._leave_masks()
         dtype, _ = self.native.arrays[f"proj{k}__{name}"]
         data = to_bf16(arr) if dtype == np.uint16 else np.asarray(arr, dtype=dtype)
         self.native.write(f"proj{k}__{name}", data)

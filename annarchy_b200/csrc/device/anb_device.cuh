@@ -1270,6 +1270,42 @@ __device__ __forceinline__ R anb_mask_add(R g, R w, const anb_u32* list, int n) 
   }
   return g;
 }
+// The same with one delay per synapse: for every listed mask with this lane's
+// bit, one event more for the step its delay names (delays: this lane's column
+// of the matrix, `stride` bytes per row; cnt: this lane's counters, `stride`
+// per step, in a ring of `slots`; `from`: the slot of the emission step). A
+// delay below `least` has arrived before the run began.
+__device__ __forceinline__ void anb_mask_delays(const anb_u32* list, const anb_u32* rows, int n,
+                                                const unsigned char* __restrict__ delays, int stride,
+                                                unsigned short* cnt, int from, int slots, int least) {
+  const anb_u32 bit = 1u << (threadIdx.x & 31);
+#pragma unroll 1
+  for (int k = 0; k < n; k += 4) {
+    const uint4 v = *reinterpret_cast<const uint4*>(list + k);
+    const uint4 r = *reinterpret_cast<const uint4*>(rows + k);
+    const anb_u32 m[4] = {v.x, v.y, v.z, v.w}, q[4] = {r.x, r.y, r.z, r.w};
+    int d[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) d[u] = (m[u] & bit) ? (int)delays[(size_t)q[u] * stride] : 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (d[u] > 0 && d[u] >= least) {
+        const int at = from + d[u];
+        cnt[(at >= slots ? at - slots : at) * stride] += 1;
+      }
+  }
+}
+// g plus w as often as counted; the counter starts again.
+template <typename R>
+__device__ __forceinline__ R anb_mask_drain(R g, R w, unsigned short* cnt) {
+  int c = *cnt;
+  if (c) *cnt = 0;
+  while (__any_sync(0xffffffffu, c > 0)) {
+    if (c > 0) g += w;
+    --c;
+  }
+  return g;
+}
 // Store of one word into another CTA of the cluster, counted on that CTA's
 // mbarrier (launches with a cluster only; the own CTA's word is an ordinary
 // store).

@@ -20,6 +20,16 @@ weight. A step of a warp:
      and send it to every other CTA (st.async: the bytes land and are counted
      in one trip).
 
+Synaptic delays (the network is the grid engine's by name, and keeps its
+arrays): a lane counts, per projection, the events that arrive in each of the
+coming steps (16 bits per neuron and step, all of one weight), and adds the
+weight as often as counted when the step comes. Delays per synapse are a byte
+per pair of neurons in global memory (9 MB in L2 for 3000 neurons). The spike
+history stays in memory as the other engines keep it; a run begins by going
+through the steps whose spikes may still be on their way, so delays, times and
+states set between runs act as they do there. Weights that become different
+send the network to the grid engine's plan.
+
 No CTA or cluster barrier in the loop: a warp that has received all words of
 step s knows that every warp has finished reading those of step s - 1, so two
 copies of the bitmaps (by step parity) are enough. What bounds a step is this
@@ -32,7 +42,11 @@ Measured per step against the form with a cluster barrier per step and the
 synapses listed per pre-synaptic neuron (CodeGenerator.cluster_module, which
 remains for projections with several weights and for larger populations): 4000
 neurons, 8 spikes per step 1.19 us (2.56) in double and 0.99 us (1.69) in single
-precision; 1000 neurons 0.66 and 0.46 us; 400 neurons 0.62 and 0.44 us.
+precision; 1000 neurons 0.66 and 0.46 us; 400 neurons 0.62 and 0.44 us. With delays, against
+the grid engine's launches per step: 3000 neurons, 1 to 20 steps per synapse,
+2.2 us (8.3) in double precision; 400 neurons, uniform, 1.2 (7.4) in double and
+0.8 (5.6) in single precision. Runs of one step take 95 to 130 us with the wait
+(144 to 146 us through the plan), so every run length gains.
 """
 from __future__ import annotations
 
@@ -60,6 +74,9 @@ class Masks:
             d = p._csr.data
             if d.size and not np.all(d == d[0]):
                 return False
+            # (a mask has one bit per pair of neurons)
+            if any(np.unique(x).size != np.size(x) for x in (p.pre_ranks, p.post_ranks_view)):
+                return False
         return True
 
     def slots(self):
@@ -84,6 +101,9 @@ class Masks:
         """Shared memory of a CTA of a C-CTA cluster, or None."""
         a16 = lambda x: (int(x) + 15) // 16 * 16
         off, lay = 64, {"pop": {}, "slots": self.slots()}             # two mbarriers first
+        # with delays: counters of the events arriving in the next steps
+        delayed = any(p.max_delay > 1 for p in self.net.projections)
+        lay["S"] = S = max(self.c.slots.values()) + 1 if delayed else 0
         for pop in self.net.populations:
             chunk = -(-(-(-pop.size // C)) // 32) * 32
             words = (pop.size + 31) // 32
@@ -92,6 +112,11 @@ class Masks:
             for _ in (0, 1):
                 d["rep"].append(off)
                 off += a16(per * 32 * 4)
+            # with delays: the steps before the run
+            ring = self.c.slots.get(pop.id, 1)
+            d["hist"] = off
+            if ring > 1:
+                off += a16(ring * words * 4)
             lay["pop"][pop.id] = d
         lay["block"] = max(d["chunk"] for d in lay["pop"].values())
         if lay["block"] > 1024:
@@ -104,7 +129,9 @@ class Masks:
             s["off"], off = off, off + a16(s["rows"] * s["warps"] * 4)
             # per warp and projection, the masks of one round
             s["cap"] = lay["pop"][s["pre"].id]["per"] * 32 + 4
-            s["list"], off = off, off + 4 * s["cap"] * len(s["projs"]) * s["warps"]
+            s["lists"] = len(s["projs"]) * (2 if any(p._delay_steps is not None for p, _, _ in s["projs"]) else 1)
+            s["list"], off = off, off + 4 * s["cap"] * s["lists"] * s["warps"]
+            s["cnt"], off = off, off + a16(2 * S * 32 * s["warps"] * len(s["projs"]))
         lay["smem"] = off
         return lay if off <= SMEM_LIMIT else None
 
@@ -140,8 +167,46 @@ class Masks:
             for proj, _, _ in s["projs"]:
                 w = proj._csr.data
                 nat.create(f"proj{proj.id}__mw", self.c._w(np.array([w[0] if w.size else 0.0])))
+                if proj._delay_steps is not None:
+                    nat.create(f"proj{proj.id}__dm", self.delays(proj, s, lay))
+        self.lay = lay
+
+    def delays(self, proj, slot, lay):
+        """(C x rows x chunk) delays of a projection's synapses (steps, one
+        byte each; at most 63)."""
+        chunk = lay["pop"][slot["post"].id]["chunk"]
+        post_rank, row_ptr, cols, _ = proj.csr_population_ranks()
+        post = np.repeat(post_rank, np.diff(row_ptr)).astype(np.int64)
+        d = np.zeros(lay["C"] * slot["rows"] * chunk, dtype=np.uint8)
+        d[((post // chunk) * slot["rows"] + (cols - 32 * slot["w0"])) * chunk + post % chunk] = proj._delay_steps
+        return d
+
+    def write_delays(self, proj):
+        """The delays set after compile() (uniform ones are read from their
+        array at the start of a run)."""
+        for s in self.lay["slots"]:
+            if proj._delay_steps is not None and any(q is proj for q, _, _ in s["projs"]):
+                self.c.native.write(f"proj{proj.id}__dm", self.delays(proj, s, self.lay))
+
+    def write_weights(self, proj) -> bool:
+        """The weights set after compile(); False when they differ."""
+        w = proj._csr.data
+        if not np.all(w == w[0]):
+            return False
+        self.c.native.write(f"proj{proj.id}__mw", self.c._w(np.array([w[0]])))
+        return True
 
     def module(self, lay) -> Module:
+        # (the update code of a kernel that neither lists spikes nor has inboxes)
+        c = self.c
+        lists, inbox = c.spike_lists, c.inbox
+        c.spike_lists, c.inbox = False, set()
+        try:
+            return self._module(lay, lists)
+        finally:
+            c.spike_lists, c.inbox = lists, inbox
+
+    def _module(self, lay, lists: bool) -> Module:
         c, net = self.c, self.net
         gen = CodeGenerator(c)
         R, C, block = gen.real, lay["C"], lay["block"]
@@ -154,10 +219,22 @@ class Masks:
                        f"anb_u32* const anb_rep{k}0 = reinterpret_cast<anb_u32*>(anb_smem + {d['rep'][0]});",
                        f"anb_u32* const anb_rep{k}1 = reinterpret_cast<anb_u32*>(anb_smem + {d['rep'][1]});"]
             spk = gen.ptr(f"pop{k}__spk")
+            ring = c.slots.get(k, 1)
+            # the spikes before the run are read from the bitmaps in memory
+            last = f"{spk} + (size_t)anb_ring_slot(t0 - 1, {ring}) * {d['words']}"
             load.append(f"#pragma unroll 1\n    for (int q = threadIdx.x; q < {32 * d['per']}; q += {block}) {{ "
-                        f"anb_rep{k}1[q] = q < {d['words']} ? {spk}[q] : 0u; anb_rep{k}0[q] = 0u; }}")
-            store.append(f"if (anb_tid < anb_cnt{k} && anb_lane == 0) {spk}[(anb_base{k} + anb_tid) >> 5] = "
-                         f"(nsteps & 1 ? anb_rep{k}0 : anb_rep{k}1)[(anb_base{k} + anb_tid) >> 5];")
+                        f"anb_rep{k}1[q] = q < {d['words']} ? ({last})[q] : 0u; anb_rep{k}0[q] = 0u; }}")
+            if ring > 1:
+                load.append(f"#pragma unroll 4\n    for (int q = threadIdx.x; q < {ring * d['words']}; q += {block}) "
+                            f"reinterpret_cast<anb_u32*>(anb_smem + {d['hist']})[q] = {spk}[q];")
+            if lists and lay["S"]:
+                # (the grid engine's spike lists are emptied when the time is set)
+                spn = gen.ptr(f"pop{k}__spn")
+                regs.append(f"const bool anb_had{k} = {spn}[(t0 - 1) & 1] != 0;")
+                store.append(f"if (anb_rank == 0 && threadIdx.x < 2) {spn}[threadIdx.x] = 1;")
+            if ring == 1:
+                store.append(f"if (anb_tid < anb_cnt{k} && anb_lane == 0) {spk}[(anb_base{k} + anb_tid) >> 5] = "
+                             f"(nsteps & 1 ? anb_rep{k}0 : anb_rep{k}1)[(anb_base{k} + anb_tid) >> 5];")
             smem = {}
             names = [(n, R) for n in c._local_vars(pop)] + [("refractory_remaining", "int")]
             if pop._has_refractory:
@@ -183,46 +260,108 @@ class Masks:
                         f"{gen.ptr(f'net__masks{i}')}[(size_t)anb_rank * {n4} + q];")
             regs.append(f"const anb_u32* const anb_mask{i} = reinterpret_cast<const anb_u32*>(anb_smem + {s['off']}) + anb_warp;")
             regs.append(f"anb_u32* const anb_li{i} = reinterpret_cast<anb_u32*>(anb_smem + {s['list']}) + "
-                        f"anb_warp * {s['cap'] * len(s['projs'])};")
-            pack, adds = "", ""
+                        f"anb_warp * {s['cap'] * s['lists']};")
+            S, chunk = lay["S"], lay["pop"][b]["chunk"]
+            if S:
+                n2 = S * chunk * len(s["projs"])
+                load.append(f"#pragma unroll 1\n    for (int q = threadIdx.x; q < {n2}; q += {block}) "
+                            f"reinterpret_cast<unsigned short*>(anb_smem + {s['cnt']})[q] = 0;")
+            pack, adds, drain = "", "", ""
             for q, (proj, w0, w1) in enumerate(s["projs"]):
-                regs.append(f"const {R} anb_w{proj.id} = ({R})anb_wf({gen.ptr(f'proj{proj.id}__mw')}[0]);")
+                pk = proj.id
+                regs.append(f"const {R} anb_w{pk} = ({R})anb_wf({gen.ptr(f'proj{pk}__mw')}[0]);")
                 at = f"anb_li{i} + {q * s['cap']}"
+                rows = f"anb_li{i} + {(len(s['projs']) + q) * s['cap']}"
+                synapse = proj._delay_steps is not None
                 pack += f"""
             int anb_n{q} = 0;"""
                 for j in range(w0 // 32, (w1 - 1) // 32 + 1):
                     # (words outside the projection's range belong to others)
                     inside = "" if w0 <= 32 * j and 32 * j + 32 <= w1 else \
                         f" && anb_lane >= {max(0, w0 - 32 * j)} && anb_lane < {min(32, w1 - 32 * j)}"
+                    if synapse:
+                        pack += f"""
+            {{ int n = anb_n{q}; anb_pack((anb_u32)anb_r[{j}], anb_m[{j}] != 0u{inside}, {rows}, &n); }}"""
                     pack += f"""
             anb_pack(anb_m[{j}], anb_m[{j}] != 0u{inside}, {at}, &anb_n{q});"""
                 pack += f"""
             if (anb_lane < 4) ({at})[anb_n{q} + anb_lane] = 0u;"""
-                adds += f"""
-            anb_rg{b}_g_{proj.target} = anb_mask_add(anb_rg{b}_g_{proj.target}, anb_w{proj.id}, {at}, anb_n{q});  // {proj.name}"""
+                if synapse:
+                    pack += f"""
+            if (anb_lane < 4) ({rows})[anb_n{q} + anb_lane] = 0u;"""
+                g = f"anb_rg{b}_g_{proj.target}"
+                if not S:
+                    adds += f"""
+            {g} = anb_mask_add({g}, anb_w{pk}, {at}, anb_n{q});  // {proj.name}"""
+                    continue
+                cnt = f"anb_cn{i} + {q * S * chunk}"
+                if synapse:
+                    adds += f"""
+            anb_mask_delays({at}, {rows}, anb_n{q}, {gen.ptr(f'proj{pk}__dm')} + (size_t)anb_rank * {s['rows'] * chunk} + anb_tid,
+                            {chunk}, {cnt}, anb_cur - 1, {S}, 1 - anb_s);  // {proj.name}"""
+                else:
+                    least = "1 - anb_s"
+                    if proj.max_delay > 1:
+                        regs.append(f"const int anb_d{pk} = {gen.ptr(f'proj{pk}__delay')}[0];")
+                    else:
+                        regs.append(f"const int anb_d{pk} = 1;")
+                        if lists:
+                            least = f"(anb_s > 0 || anb_had{a} ? 1 - anb_s : 2)"
+                    adds += f"""
+            if (anb_d{pk} >= {least}) {{  // {proj.name}
+              const int c = anb_mask_add(0, 1, {at}, anb_n{q}), at = anb_cur - 1 + anb_d{pk};
+              if (c) ({cnt})[(at >= {S} ? at - {S} : at) * {chunk}] += (unsigned short)c;
+            }}"""
+                drain += f"""
+          {g} = anb_mask_drain({g}, anb_w{pk}, {cnt} + anb_cur * {chunk});  // {proj.name}"""
+            if S:
+                regs.append(f"unsigned short* const anb_cn{i} = reinterpret_cast<unsigned short*>(anb_smem + {s['cnt']}) + anb_tid;")
             word = "anb_rep[j * 32 + anb_lane]"
             used = [(w0, w1) for _, w0, w1 in s["projs"]]
             if len(used) != 1 or used[0] != (0, lay["pop"][a]["words"]):
                 word = " || ".join(f"(j * 32 + anb_lane >= {w0} && j * 32 + anb_lane < {w1})"
                                    for w0, w1 in used) + " ? " + word + " : 0u"
             any_x = " | ".join(f"anb_x[{j}]" for j in range(per))
+            by_row = s["lists"] > len(s["projs"])
+            rowdecl = f"\n          int anb_r[{per}];" if by_row else ""
+            rowset = (f"anb_r[j] = (j * 32 + anb_lane) * 32 + __ffs(anb_x[j]) - {s['w0'] * 32 + 1};\n              "
+                      if by_row else "")
+            if drain:
+                drain = f"""
+          if (anb_s >= 0) {{{drain}
+          }}"""
+            ring, words = c.slots.get(a, 1), lay["pop"][a]["words"]
+            inside = " || ".join(f"(i >= {w0} && i < {w1})" for w0, w1 in used)
+            history = f"-anb_s < {ring} && ({inside}) ? anb_hist[i] : 0u" if ring > 1 else "0u"
+            earlier = f"""
+          if (anb_s < 0) {{
+            // steps before the run: spikes still on their way
+            const anb_u32* anb_hist = reinterpret_cast<const anb_u32*>(anb_smem + {lay['pop'][a]['hist']}) +
+                                      anb_ring_slot(t - 1, {ring}) * {words};
+            (void)anb_hist;
+#pragma unroll
+            for (int j = 0; j < {per}; ++j) {{
+              const int i = j * 32 + anb_lane;
+              anb_x[j] = {history};
+            }}
+          }}""" if lay["S"] else ""
             deliver += f"""
         if (anb_warp < {s['warps']}) {{  // population {a}'s spikes of the previous step (word j * 32 + lane: lane's j-th)
           const anb_u32* anb_rep = (anb_s & 1) ? anb_rep{a}0 : anb_rep{a}1;
-          anb_u32 anb_x[{per}], anb_m[{per}];
+          anb_u32 anb_x[{per}], anb_m[{per}];{rowdecl}
 #pragma unroll
-          for (int j = 0; j < {per}; ++j) anb_x[j] = {word};
+          for (int j = 0; j < {per}; ++j) anb_x[j] = {word};{earlier}
 #pragma unroll 1
           while (__any_sync(0xffffffffu, ({any_x}) != 0u)) {{
             // the mask of each word's first spike
 #pragma unroll
             for (int j = 0; j < {per}; ++j) {{
               anb_m[j] = anb_x[j] ? anb_mask{i}[((j * 32 + anb_lane) * 32 + __ffs(anb_x[j]) - {s['w0'] * 32 + 1}) * {s['warps']}] : 0u;
-              anb_x[j] &= anb_x[j] - 1u;
+              {rowset}anb_x[j] &= anb_x[j] - 1u;
             }}{pack}
             __syncwarp();{adds}
             __syncwarp();
-          }}
+          }}{drain}
         }}"""
         globals_ = [gen._globals_preamble(p, lambda n, kk=p.id: gen.ptr(f"pop{kk}__{n}")) for p in net.populations]
         mon_pre = "\n    ".join(
@@ -234,6 +373,13 @@ class Masks:
         warps = f"anb_cnt{net.populations[0].id}"
         for p in net.populations[1:]:
             warps = f"max({warps}, anb_cnt{p.id})"
+        # with delays the steps before the run that still matter come first
+        S = lay["S"]
+        start = f"nsteps > 0 ? {2 - S} : 0" if S else "0"
+        cursor = f"""
+        const int anb_cur = anb_ring_slot(t, {S});""" if S else ""
+        skip = """
+        if (anb_s < 0) continue;""" if S else ""
         own = " + ".join(f"(anb_cnt{p.id} + 31) / 32" for p in net.populations)
         nl = "\n    "
         err = gen.ptr("err")
@@ -266,14 +412,14 @@ extern "C" __global__ void __launch_bounds__({block}, 1) anb_cluster_run(long lo
     // (warps without neurons send nothing, so nobody waits for them: they stay out)
     if (anb_warp < anb_warps) {{
 #pragma unroll 1
-      for (int anb_s = 0; anb_s < nsteps; ++anb_s) {{
-        const long long t = t0 + anb_s;
+      for (int anb_s = {start}; anb_s < nsteps; ++anb_s) {{
+        const long long t = t0 + anb_s;{cursor}
         if (anb_s > 0) {{
           // the words of step s - 1; the barrier's next phase takes those of s + 1
           const unsigned b = anb_bar + 8u * ((anb_s - 1) & 1);
           if (!anb_mbar_wait(b, ((anb_s - 1) >> 1) & 1, {err})) break;
           if (threadIdx.x == 0) anb_mbar_expect(b, anb_bytes);
-        }}{deliver}
+        }}{deliver}{skip}
         {''.join(ups)}
         __syncwarp();
         if (anb_lane == 0) anb_mbar_arrive(anb_bar + 8u * (anb_s & 1));
@@ -295,7 +441,12 @@ extern "C" __global__ void __launch_bounds__({block}, 1) anb_cluster_run(long lo
         send = "" if lay["C"] == 1 else f"""
           if (anb_lane != (int)anb_rank && anb_lane < {lay['C']})
             anb_st_async(anb_peer + anb_off, anb_m, anb_peer + 8u * (anb_s & 1));"""
-        rec = ""
+        rec, keep, ring = "", "", self.c.slots.get(k, 1)
+        if ring > 1:
+            # the history ring in memory, as the other engines keep it
+            keep = f"""
+          if (anb_lane == 30)
+            {gen.ptr(f'pop{k}__spk')}[(size_t)anb_ring_slot(t, {ring}) * {d['words']} + ((unsigned)(anb_base + anb_q) >> 5)] = anb_m;"""
         for m in self.net.monitors:
             if m.population is pop and "spike" in m.variables:
                 ml = self.c.mon_layout[m.id]
@@ -312,7 +463,7 @@ extern "C" __global__ void __launch_bounds__({block}, 1) anb_cluster_run(long lo
         const anb_u32 anb_m = __ballot_sync(0xffffffffu, anb_spiked);
         if (anb_q - anb_lane < anb_cnt) {{
           const unsigned anb_off = ((anb_s & 1) ? {d['rep'][1]}u : {d['rep'][0]}u) + 4u * (unsigned)((anb_base + anb_q) >> 5);
-          if (anb_lane == (int)anb_rank) *reinterpret_cast<anb_u32*>(anb_smem + anb_off) = anb_m;{send}{rec}
+          if (anb_lane == (int)anb_rank) *reinterpret_cast<anb_u32*>(anb_smem + anb_off) = anb_m;{send}{keep}{rec}
         }}
       }}"""
         code = gen.neuron_update(pop, local_engine=True, smem=smem, cluster={}, ballot_hook=hook)
