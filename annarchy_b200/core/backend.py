@@ -221,7 +221,7 @@ class CompiledNetwork:
                 or self.net._config.get("persistent") or not self._local_possible(delays=True)[0]):
             return None
         masks = Masks(self)
-        return masks if masks.possible() and masks.choose() else None
+        return masks if masks.possible() else None
 
     def _load_masks(self, masks) -> bool:
         from ..runtime.lib import BackendError

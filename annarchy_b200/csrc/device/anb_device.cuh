@@ -1271,27 +1271,42 @@ __device__ __forceinline__ R anb_mask_add(R g, R w, const anb_u32* list, int n) 
   return g;
 }
 // The same with one delay per synapse: for every listed mask with this lane's
-// bit, one event more for the step its delay names (delays: this lane's column
-// of the matrix, `stride` bytes per row; cnt: this lane's counters, `stride`
-// per step, in a ring of `slots`; `from`: the slot of the emission step). A
-// delay below `least` has arrived before the run began.
-__device__ __forceinline__ void anb_mask_delays(const anb_u32* list, const anb_u32* rows, int n,
-                                                const unsigned char* __restrict__ delays, int stride,
-                                                unsigned short* cnt, int from, int slots, int least) {
-  const anb_u32 bit = 1u << (threadIdx.x & 31);
+// bit, one event more for the step its delay names. at[k]: the projection << 24
+// plus the position of the delays: of the first of the mask's synapses (PACKED),
+// or the row of a matrix whose column of this lane `delays` is (`stride` bytes
+// per row). cnt: 16-bit counters, `chunk` per step in a ring of `slots`,
+// `proj_size` per projection; `from`: the slot of the emission step. A delay
+// below `least` has arrived before the run began. The counters take an atomic
+// without a result: nothing waits for it (load, add and store one after another
+// were 35 cycles per mask).
+template <bool PACKED>
+__device__ __forceinline__ void anb_mask_delays(const anb_u32* list, const anb_u32* at, int n,
+                                                const unsigned char* delays, int stride, anb_u32* cnt,
+                                                int proj_size, int chunk, int from, int slots, int least) {
+  constexpr int U = PACKED ? 4 : 8;         // (a matrix in global memory: more loads under way)
+  const int lane = threadIdx.x & 31;
+  const anb_u32 bit = 1u << lane, below = bit - 1u, one = (lane & 1) ? 0x10000u : 1u;
 #pragma unroll 1
-  for (int k = 0; k < n; k += 4) {
-    const uint4 v = *reinterpret_cast<const uint4*>(list + k);
-    const uint4 r = *reinterpret_cast<const uint4*>(rows + k);
-    const anb_u32 m[4] = {v.x, v.y, v.z, v.w}, q[4] = {r.x, r.y, r.z, r.w};
-    int d[4];
+  for (int k = 0; k < n; k += U) {
+    anb_u32 m[U], q[U];
+    int d[U];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) d[u] = (m[u] & bit) ? (int)delays[(size_t)q[u] * stride] : 0;
+    for (int u = 0; u < U; u += 4) {
+      const uint4 v = *reinterpret_cast<const uint4*>(list + k + u);
+      const uint4 r = *reinterpret_cast<const uint4*>(at + k + u);
+      m[u] = v.x; m[u + 1] = v.y; m[u + 2] = v.z; m[u + 3] = v.w;
+      q[u] = r.x; q[u + 1] = r.y; q[u + 2] = r.z; q[u + 3] = r.w;
+    }
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < U; ++u) {
+      const anb_u32 p = q[u] & 0xffffffu;
+      d[u] = !(m[u] & bit) ? 0 : PACKED ? (int)delays[p + __popc(m[u] & below)] : (int)delays[(size_t)p * stride];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
       if (d[u] > 0 && d[u] >= least) {
-        const int at = from + d[u];
-        cnt[(at >= slots ? at - slots : at) * stride] += 1;
+        const int s = from + d[u] >= slots ? from + d[u] - slots : from + d[u];
+        atomicAdd(cnt + ((int)(q[u] >> 24) * proj_size + s * chunk + (int)threadIdx.x) / 2, one);
       }
   }
 }
@@ -1300,10 +1315,10 @@ template <typename R>
 __device__ __forceinline__ R anb_mask_drain(R g, R w, unsigned short* cnt) {
   int c = *cnt;
   if (c) *cnt = 0;
-  while (__any_sync(0xffffffffu, c > 0)) {
+  if (c > 0) g += w;                        // (mostly none or one: no vote to wait for)
+  if (c > 1) g += w;
+  for (c -= 2; __any_sync(0xffffffffu, c > 0); --c)
     if (c > 0) g += w;
-    --c;
-  }
   return g;
 }
 // Store of one word into another CTA of the cluster, counted on that CTA's

@@ -23,8 +23,10 @@ weight. A step of a warp:
 Synaptic delays (the network is the grid engine's by name, and keeps its
 arrays): a lane counts, per projection, the events that arrive in each of the
 coming steps (16 bits per neuron and step, all of one weight), and adds the
-weight as often as counted when the step comes. Delays per synapse are a byte
-per pair of neurons in global memory (9 MB in L2 for 3000 neurons). The spike
+weight as often as counted when the step comes. Delays per synapse lie next to
+the masks, one byte per synapse, found by the first position of a row's warp
+and the mask's bits below the lane's; where they do not fit, a byte per pair of
+neurons in global memory (14 MB, in L2, for 4000 neurons on 16 CTAs). The spike
 history stays in memory as the other engines keep it; a run begins by going
 through the steps whose spikes may still be on their way, so delays, times and
 states set between runs act as they do there. Weights that become different
@@ -44,8 +46,9 @@ remains for projections with several weights and for larger populations): 4000
 neurons, 8 spikes per step 1.19 us (2.56) in double and 0.99 us (1.69) in single
 precision; 1000 neurons 0.66 and 0.46 us; 400 neurons 0.62 and 0.44 us. With delays, against
 the grid engine's launches per step: 3000 neurons, 1 to 20 steps per synapse,
-2.2 us (8.3) in double precision; 400 neurons, uniform, 1.2 (7.4) in double and
-0.8 (5.6) in single precision. Runs of one step take 95 to 130 us with the wait
+1.8 us (9.4) in double precision (2.0 with the delays in global memory and a
+list per projection); 400 neurons, uniform, 1.1 (7.4) in double and 0.7 (5.4) in
+single precision. Runs of one step take 95 to 130 us with the wait
 (144 to 146 us through the plan), so every run length gains.
 """
 from __future__ import annotations
@@ -128,12 +131,27 @@ class Masks:
             s["rows"] = (s["w1"] - s["w0"]) * 32
             s["off"], off = off, off + a16(s["rows"] * s["warps"] * 4)
             # per warp and projection, the masks of one round
-            s["cap"] = lay["pop"][s["pre"].id]["per"] * 32 + 4
-            s["lists"] = len(s["projs"]) * (2 if any(p._delay_steps is not None for p, _, _ in s["projs"]) else 1)
+            s["cap"] = lay["pop"][s["pre"].id]["per"] * 32 + 8
+            # (one list, with the positions of the delays, for all projections with delays per synapse)
+            s["synapse"] = [q for q, (p, _, _) in enumerate(s["projs"]) if p._delay_steps is not None]
+            s["lists"] = len(s["projs"]) - len(s["synapse"]) + (2 if s["synapse"] else 0)
             s["list"], off = off, off + 4 * s["cap"] * s["lists"] * s["warps"]
             s["cnt"], off = off, off + a16(2 * S * 32 * s["warps"] * len(s["projs"]))
+        if off > SMEM_LIMIT:
+            return None
+        for s in lay["slots"]:
+            # the delays of the synapses next to the masks, where they fit
+            s["packed"] = False
+            if s["synapse"]:
+                positions, delays = self.packed(s, lay)
+                n = delays.shape[1]
+                more = a16(positions.shape[1] * 2) + a16(n)
+                if n < 65536 and off + more <= SMEM_LIMIT:
+                    s["packed"], s["nbytes"], s["arrays"] = True, n, (positions, delays)
+                    s["pos"], off = off, off + a16(positions.shape[1] * 2)
+                    s["bytes"], off = off, off + a16(n)
         lay["smem"] = off
-        return lay if off <= SMEM_LIMIT else None
+        return lay
 
     def choose(self):
         """Layouts to try, the preferred one first: about 128 neurons per CTA
@@ -145,8 +163,8 @@ class Masks:
         else:
             total = max(p.size for p in self.net.populations)
             first = next((c for c in (1, 2, 4, 8) if total <= 128 * c), 16)
-            lays = [self.layout(c) for c in (1, 2, 4, 8, 16) if c >= first]
-        return [x for x in lays if x]
+            lays = (self.layout(c) for c in (1, 2, 4, 8, 16) if c >= first)
+        return (x for x in lays if x)
 
     def tables(self, slot, lay):
         """(C x rows x warps) masks of a table."""
@@ -167,26 +185,57 @@ class Masks:
             for proj, _, _ in s["projs"]:
                 w = proj._csr.data
                 nat.create(f"proj{proj.id}__mw", self.c._w(np.array([w[0] if w.size else 0.0])))
-                if proj._delay_steps is not None:
-                    nat.create(f"proj{proj.id}__dm", self.delays(proj, s, lay))
+            self._delay_arrays(i, s, lay, nat.create)
         self.lay = lay
 
-    def delays(self, proj, slot, lay):
-        """(C x rows x chunk) delays of a projection's synapses (steps, one
-        byte each; at most 63)."""
-        chunk = lay["pop"][slot["post"].id]["chunk"]
-        post_rank, row_ptr, cols, _ = proj.csr_population_ranks()
-        post = np.repeat(post_rank, np.diff(row_ptr)).astype(np.int64)
-        d = np.zeros(lay["C"] * slot["rows"] * chunk, dtype=np.uint8)
-        d[((post // chunk) * slot["rows"] + (cols - 32 * slot["w0"])) * chunk + post % chunk] = proj._delay_steps
+    def _delay_arrays(self, i, slot, lay, put):
+        if slot["packed"]:
+            positions, delays = slot.pop("arrays", None) or self.packed(slot, lay)
+            put(f"net__dpos{i}", positions.reshape(-1))
+            put(f"net__dby{i}", delays.reshape(-1))
+        elif slot["synapse"]:
+            put(f"net__dby{i}", self.delays(slot, lay))
+
+    def _synapses(self, slot, lay):
+        """((CTA x row x lane) index, delay) of the synapses of a table's
+        projections with delays per synapse."""
+        chunk, at, steps = lay["pop"][slot["post"].id]["chunk"], [], []
+        for q in slot["synapse"]:
+            proj = slot["projs"][q][0]
+            post_rank, row_ptr, cols, _ = proj.csr_population_ranks()
+            post = np.repeat(post_rank, np.diff(row_ptr)).astype(np.int64)
+            at.append(((post // chunk) * slot["rows"] + (cols - 32 * slot["w0"])) * chunk + post % chunk)
+            steps.append(np.asarray(proj._delay_steps))
+        return np.concatenate(at), np.concatenate(steps)
+
+    def delays(self, slot, lay):
+        """(C x rows x chunk) delays (steps, one byte each; at most 63)."""
+        d = np.zeros(lay["C"] * slot["rows"] * lay["pop"][slot["post"].id]["chunk"], dtype=np.uint8)
+        at, steps = self._synapses(slot, lay)
+        d[at] = steps
         return d
+
+    def packed(self, slot, lay):
+        """Per CTA the first positions (rows x warps) and the delays of the
+        synapses in the order of rows and lanes."""
+        C, per = lay["C"], slot["rows"] * slot["warps"]
+        at, steps = self._synapses(slot, lay)
+        order = np.argsort(at, kind="stable")
+        count = np.bincount(at // 32, minlength=C * per).reshape(C, per)
+        total = count.sum(axis=1)
+        first = np.cumsum(count, axis=1) - count
+        d = np.zeros((C, int(total.max())), dtype=np.uint8)
+        ends = np.cumsum(total)
+        for c in range(C):
+            d[c, :total[c]] = steps[order[ends[c] - total[c]:ends[c]]]
+        return first.astype(np.uint16), d
 
     def write_delays(self, proj):
         """The delays set after compile() (uniform ones are read from their
         array at the start of a run)."""
-        for s in self.lay["slots"]:
-            if proj._delay_steps is not None and any(q is proj for q, _, _ in s["projs"]):
-                self.c.native.write(f"proj{proj.id}__dm", self.delays(proj, s, self.lay))
+        for i, s in enumerate(self.lay["slots"]):
+            if any(s["projs"][q][0] is proj for q in s["synapse"]):
+                self._delay_arrays(i, s, self.lay, self.c.native.write)
 
     def write_weights(self, proj) -> bool:
         """The weights set after compile(); False when they differ."""
@@ -266,14 +315,45 @@ class Masks:
                 n2 = S * chunk * len(s["projs"])
                 load.append(f"#pragma unroll 1\n    for (int q = threadIdx.x; q < {n2}; q += {block}) "
                             f"reinterpret_cast<unsigned short*>(anb_smem + {s['cnt']})[q] = 0;")
-            pack, adds, drain = "", "", ""
+            pack, adds, drain, place = "", "", "", ""
+            uniform = [q for q in range(len(s["projs"])) if q not in s["synapse"]]
+            if s["synapse"]:
+                dby = f"anb_li{i} + {len(uniform) * s['cap']}"
+                dat = f"anb_li{i} + {(len(uniform) + 1) * s['cap']}"
+                pack += """
+            int anb_nd = 0;"""
+                if s["packed"]:
+                    n16 = s["rows"] * s["warps"]
+                    for what, ct, at, n in (("dpos", "unsigned short", s["pos"], n16),
+                                            ("dby", "unsigned char", s["bytes"], s["nbytes"])):
+                        load.append(f"#pragma unroll 4\n    for (int q = threadIdx.x; q < {n}; q += {block}) "
+                                    f"reinterpret_cast<{ct}*>(anb_smem + {at})[q] = "
+                                    f"{gen.ptr(f'net__{what}{i}')}[(size_t)anb_rank * {n} + q];")
+                    regs.append(f"const unsigned short* const anb_dp{i} = "
+                                f"reinterpret_cast<const unsigned short*>(anb_smem + {s['pos']}) + anb_warp;")
+                    row = f"(int)anb_dp{i}[anb_row * {s['warps']}]"
+                    where = f"anb_smem + {s['bytes']}, 0"
+                else:
+                    row = "anb_row"
+                    where = f"{gen.ptr(f'net__dby{i}')} + (size_t)anb_rank * {s['rows'] * chunk} + anb_tid, {chunk}"
+                # the delays' position, and above it the projection
+                place = f"""
+              anb_r[j] = 0;
+              if (anb_m[j]) {{
+                const int anb_row = (j * 32 + anb_lane) * 32 + __ffs(anb_x[j]) - {s['w0'] * 32 + 1};
+                anb_r[j] = {row}{''.join(f" + (j * 32 + anb_lane >= {s['projs'][q][1]} && j * 32 + anb_lane < {s['projs'][q][2]} ? {q << 24} : 0)" for q in s["synapse"] if q)};
+              }}"""
+                adds += f"""
+            anb_mask_delays<{'true' if s['packed'] else 'false'}>({dby}, {dat}, anb_nd, {where},
+                            reinterpret_cast<anb_u32*>(anb_smem + {s['cnt']}), {S * chunk}, {chunk},
+                            anb_cur - 1, {S}, 1 - anb_s);"""
             for q, (proj, w0, w1) in enumerate(s["projs"]):
                 pk = proj.id
                 regs.append(f"const {R} anb_w{pk} = ({R})anb_wf({gen.ptr(f'proj{pk}__mw')}[0]);")
-                at = f"anb_li{i} + {q * s['cap']}"
-                rows = f"anb_li{i} + {(len(s['projs']) + q) * s['cap']}"
-                synapse = proj._delay_steps is not None
-                pack += f"""
+                synapse = q in s["synapse"]
+                n, at = ("anb_nd", dby) if synapse else (f"anb_n{q}", f"anb_li{i} + {uniform.index(q) * s['cap']}")
+                if not synapse:
+                    pack += f"""
             int anb_n{q} = 0;"""
                 for j in range(w0 // 32, (w1 - 1) // 32 + 1):
                     # (words outside the projection's range belong to others)
@@ -281,51 +361,47 @@ class Masks:
                         f" && anb_lane >= {max(0, w0 - 32 * j)} && anb_lane < {min(32, w1 - 32 * j)}"
                     if synapse:
                         pack += f"""
-            {{ int n = anb_n{q}; anb_pack((anb_u32)anb_r[{j}], anb_m[{j}] != 0u{inside}, {rows}, &n); }}"""
+            {{ int n = anb_nd; anb_pack((anb_u32)anb_r[{j}], anb_m[{j}] != 0u{inside}, {dat}, &n); }}"""
                     pack += f"""
-            anb_pack(anb_m[{j}], anb_m[{j}] != 0u{inside}, {at}, &anb_n{q});"""
-                pack += f"""
+            anb_pack(anb_m[{j}], anb_m[{j}] != 0u{inside}, {at}, &{n});"""
+                if not synapse:
+                    pack += f"""
             if (anb_lane < 4) ({at})[anb_n{q} + anb_lane] = 0u;"""
-                if synapse:
-                    pack += f"""
-            if (anb_lane < 4) ({rows})[anb_n{q} + anb_lane] = 0u;"""
                 g = f"anb_rg{b}_g_{proj.target}"
                 if not S:
                     adds += f"""
             {g} = anb_mask_add({g}, anb_w{pk}, {at}, anb_n{q});  // {proj.name}"""
                     continue
                 cnt = f"anb_cn{i} + {q * S * chunk}"
+                drain += f"""
+          {g} = anb_mask_drain({g}, anb_w{pk}, {cnt} + anb_cur * {chunk});  // {proj.name}"""
                 if synapse:
-                    adds += f"""
-            anb_mask_delays({at}, {rows}, anb_n{q}, {gen.ptr(f'proj{pk}__dm')} + (size_t)anb_rank * {s['rows'] * chunk} + anb_tid,
-                            {chunk}, {cnt}, anb_cur - 1, {S}, 1 - anb_s);  // {proj.name}"""
+                    continue
+                least = "1 - anb_s"
+                if proj.max_delay > 1:
+                    regs.append(f"const int anb_d{pk} = {gen.ptr(f'proj{pk}__delay')}[0];")
                 else:
-                    least = "1 - anb_s"
-                    if proj.max_delay > 1:
-                        regs.append(f"const int anb_d{pk} = {gen.ptr(f'proj{pk}__delay')}[0];")
-                    else:
-                        regs.append(f"const int anb_d{pk} = 1;")
-                        if lists:
-                            least = f"(anb_s > 0 || anb_had{a} ? 1 - anb_s : 2)"
-                    adds += f"""
+                    regs.append(f"const int anb_d{pk} = 1;")
+                    if lists:
+                        least = f"(anb_s > 0 || anb_had{a} ? 1 - anb_s : 2)"
+                adds += f"""
             if (anb_d{pk} >= {least}) {{  // {proj.name}
               const int c = anb_mask_add(0, 1, {at}, anb_n{q}), at = anb_cur - 1 + anb_d{pk};
               if (c) ({cnt})[(at >= {S} ? at - {S} : at) * {chunk}] += (unsigned short)c;
             }}"""
-                drain += f"""
-          {g} = anb_mask_drain({g}, anb_w{pk}, {cnt} + anb_cur * {chunk});  // {proj.name}"""
+            if s["synapse"]:
+                pack += f"""
+            if (anb_lane < 8) ({dby})[anb_nd + anb_lane] = 0u;
+            if (anb_lane < 8) ({dat})[anb_nd + anb_lane] = 0u;"""
             if S:
-                regs.append(f"unsigned short* const anb_cn{i} = reinterpret_cast<unsigned short*>(anb_smem + {s['cnt']}) + anb_tid;")
+                regs.append(f"unsigned short* const anb_cn{i} = reinterpret_cast<unsigned short*>(anb_smem + {s['cnt']}) + anb_tid;\n    (void)anb_cn{i};")
             word = "anb_rep[j * 32 + anb_lane]"
             used = [(w0, w1) for _, w0, w1 in s["projs"]]
             if len(used) != 1 or used[0] != (0, lay["pop"][a]["words"]):
                 word = " || ".join(f"(j * 32 + anb_lane >= {w0} && j * 32 + anb_lane < {w1})"
                                    for w0, w1 in used) + " ? " + word + " : 0u"
             any_x = " | ".join(f"anb_x[{j}]" for j in range(per))
-            by_row = s["lists"] > len(s["projs"])
-            rowdecl = f"\n          int anb_r[{per}];" if by_row else ""
-            rowset = (f"anb_r[j] = (j * 32 + anb_lane) * 32 + __ffs(anb_x[j]) - {s['w0'] * 32 + 1};\n              "
-                      if by_row else "")
+            rowdecl = f"\n          int anb_r[{per}];" if s["synapse"] else ""
             if drain:
                 drain = f"""
           if (anb_s >= 0) {{{drain}
@@ -337,7 +413,7 @@ class Masks:
           if (anb_s < 0) {{
             // steps before the run: spikes still on their way
             const anb_u32* anb_hist = reinterpret_cast<const anb_u32*>(anb_smem + {lay['pop'][a]['hist']}) +
-                                      anb_ring_slot(t - 1, {ring}) * {words};
+                                      {f'(anb_at{a} == 0 ? {ring - 1} : anb_at{a} - 1)' if ring > 1 else '0'} * {words};
             (void)anb_hist;
 #pragma unroll
             for (int j = 0; j < {per}; ++j) {{
@@ -356,8 +432,8 @@ class Masks:
             // the mask of each word's first spike
 #pragma unroll
             for (int j = 0; j < {per}; ++j) {{
-              anb_m[j] = anb_x[j] ? anb_mask{i}[((j * 32 + anb_lane) * 32 + __ffs(anb_x[j]) - {s['w0'] * 32 + 1}) * {s['warps']}] : 0u;
-              {rowset}anb_x[j] &= anb_x[j] - 1u;
+              anb_m[j] = anb_x[j] ? anb_mask{i}[((j * 32 + anb_lane) * 32 + __ffs(anb_x[j]) - {s['w0'] * 32 + 1}) * {s['warps']}] : 0u;{place}
+              anb_x[j] &= anb_x[j] - 1u;
             }}{pack}
             __syncwarp();{adds}
             __syncwarp();
@@ -376,8 +452,16 @@ class Masks:
         # with delays the steps before the run that still matter come first
         S = lay["S"]
         start = f"nsteps > 0 ? {2 - S} : 0" if S else "0"
+        # (positions in the rings are counted: a 64-bit remainder is 100 cycles)
         cursor = f"""
-        const int anb_cur = anb_ring_slot(t, {S});""" if S else ""
+        anb_cur = anb_cur + 1 == {S} ? 0 : anb_cur + 1;""" if S else ""
+        rings = f"int anb_cur = anb_ring_slot(t0 + ({start}) - 1, {S});" if S else ""
+        for pop in net.populations:
+            ring = c.slots.get(pop.id, 1)
+            if ring > 1:
+                rings += f"\n      int anb_at{pop.id} = anb_ring_slot(t0 + ({start}) - 1, {ring});"
+                cursor += f"""
+        anb_at{pop.id} = anb_at{pop.id} + 1 == {ring} ? 0 : anb_at{pop.id} + 1;"""
         skip = """
         if (anb_s < 0) continue;""" if S else ""
         own = " + ".join(f"(anb_cnt{p.id} + 31) / 32" for p in net.populations)
@@ -411,6 +495,7 @@ extern "C" __global__ void __launch_bounds__({block}, 1) anb_cluster_run(long lo
     anb_cluster_sync();
     // (warps without neurons send nothing, so nobody waits for them: they stay out)
     if (anb_warp < anb_warps) {{
+      {rings}
 #pragma unroll 1
       for (int anb_s = {start}; anb_s < nsteps; ++anb_s) {{
         const long long t = t0 + anb_s;{cursor}
@@ -446,7 +531,7 @@ extern "C" __global__ void __launch_bounds__({block}, 1) anb_cluster_run(long lo
             # the history ring in memory, as the other engines keep it
             keep = f"""
           if (anb_lane == 30)
-            {gen.ptr(f'pop{k}__spk')}[(size_t)anb_ring_slot(t, {ring}) * {d['words']} + ((unsigned)(anb_base + anb_q) >> 5)] = anb_m;"""
+            {gen.ptr(f'pop{k}__spk')}[anb_at{k} * {d['words']} + ((anb_base + anb_q) >> 5)] = anb_m;"""
         for m in self.net.monitors:
             if m.population is pop and "spike" in m.variables:
                 ml = self.c.mon_layout[m.id]
