@@ -1040,6 +1040,26 @@ __device__ __noinline__ int anb_list_spikes(int* list, const anb_u32* bits, int 
   return n;
 }
 
+// The same from bounds that each thread has loaded beforehand (thread i: neuron
+// i of the CTA's words; lane q holds word q, zero beyond): no load between the
+// spikes and their synapses. Every warp counts for itself.
+__device__ __forceinline__ int anb_list_ranges(int* list, anb_u32 words, int neuron, int beg, int end) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = __popc(words);
+  const int n = __reduce_add_sync(0xffffffffu, c);
+  const int before = __reduce_add_sync(0xffffffffu, lane < warp ? c : 0);
+  const anb_u32 own = __shfl_sync(0xffffffffu, words, warp);
+  if ((own >> lane) & 1u) {
+    const int k = before + __popc(own & ((1u << lane) - 1u));
+    list[k] = neuron;
+    list[ANB_DELIVER_LIST + k] = 0;
+    list[2 * ANB_DELIVER_LIST + k] = beg;
+    list[3 * ANB_DELIVER_LIST + k] = end;
+  }
+  __syncthreads();
+  return n;
+}
+
 // Runs body(neuron, tag, q) for every synapse q of the n listed neurons. All
 // warps of the CTA share the synapses of a single spike, n of nwarps or more
 // get one warp each, so that few loads wait for one another.
@@ -1102,6 +1122,19 @@ __device__ __forceinline__ R anb_inbox_add(R g, anb_u32 c, const K* __restrict__
   const K* __restrict__ e = entry + (size_t)i * ANB_INBOX;
   if (c == 1u) return g + w[(anb_u32)e[0]];
   return c ? anb_inbox_sorted<R, K>(g, c, e, w) : g;
+}
+
+// The first two entries of neuron i's inbox.
+__device__ __forceinline__ void anb_inbox_first(const anb_u32* __restrict__ entry, int i, anb_u32& a, anb_u32& b) {
+  const uint2 e = *reinterpret_cast<const uint2*>(entry + (size_t)i * ANB_INBOX);
+  a = e.x;
+  b = e.y;
+}
+__device__ __forceinline__ void anb_inbox_first(const unsigned long long* __restrict__ entry, int i,
+                                                unsigned long long& a, unsigned long long& b) {
+  const ulonglong2 e = *reinterpret_cast<const ulonglong2*>(entry + (size_t)i * ANB_INBOX);
+  a = e.x;
+  b = e.y;
 }
 
 // g plus the weights w[j] of the row's synapses whose pre neuron's bit is set,

@@ -1566,6 +1566,9 @@ int anb_run(anb_net* net, int64_t nsteps) {
       remaining -= net->graph_steps;
     }
   }
+  // (what kernels read before they wait for their predecessor may have been
+  // written by the copies or kernels before this run)
+  net->pdl_prev = false;
   for (int64_t s = 0; s < remaining; ++s) {
     rc = run_plan_once(net);
     if (rc) return rc;

@@ -47,6 +47,10 @@ DEVICE_HEADER = os.path.join(os.path.dirname(HERE), "csrc", "device", "anb_devic
 BLOCK = 256
 MAX_GRID = 148 * 16
 PERSISTENT_BLOCK = 1024
+# place in a kernel's source where it waits for its predecessor on the stream:
+# above it only what no kernel writes is read (parameters, connectivity,
+# monitors' switches), while the predecessor may still run
+ENTER = "/*wait*/"
 
 CTYPE_OF = {np.dtype(np.float64): "double", np.dtype(np.float32): "float",
             np.dtype(np.int32): "int", np.dtype(np.int64): "long long",
@@ -506,7 +510,7 @@ class CodeGenerator:
             hoist.append((self.real, f"anb_kc_{x}", src))
             stores.append(f"{src}[{idx}] = anb_kc_{x};")
         K = self.neurons_per_thread(pop) if grid_path else 1
-        drain = self._inbox_drain(pop, K, loads, stores, hoist) if grid_path else ""
+        drain, entries = self._inbox_drain(pop, K, loads, stores, hoist) if grid_path else ("", "")
         if pop.neuron_type.type == "rate":
             for t in pop.targets:
                 src = gsrc("_sum_" + t)
@@ -627,7 +631,7 @@ class CodeGenerator:
       }}
     }}"""
         first = 0
-        if grid_path and K > 1:
+        if grid_path and (K > 1 or drain):
             if pop.id in getattr(self.c, "owned", {}):
                 first, size = self.c.owned[pop.id]
             derived = [ln for ln in loads if not any(ln == f"{ct} {nm} = {src}[anb_i];"
@@ -649,7 +653,7 @@ class CodeGenerator:
           if (anb_j < anb_n) {{
           {fetch}
           }}
-        }}
+        }}{entries}
 #pragma unroll
         for (int anb_k = 0; anb_k < {K}; ++anb_k) {{
         const int anb_base = anb_base0 + anb_k * blockDim.x;
@@ -688,21 +692,28 @@ class CodeGenerator:
       }}
     }}"""
 
-    def _inbox_drain(self, pop, K, loads, stores, hoist) -> str:
+    def _inbox_drain(self, pop, K, loads, stores, hoist) -> tuple[str, str]:
         """The step's increments of a neuron's conductances from its inboxes
         (inbox_projections), projection by projection, before its update; a
         neuron whose inbox ran over walks its row (the whole warp, one such
-        neuron at a time). Rewrites the update's loads of those conductances."""
+        neuron at a time). Rewrites the update's loads of those conductances.
+        Second, the code that fetches the first two entries of every inbox and
+        their weights, all projections (and neurons of the thread) at once:
+        one after another they were two dependent trips to L2 per projection."""
         R = self.real
         targets: dict = {}
         for proj in self.net.projections:
             if proj.id in self.c.inbox and proj.post_pop is pop:
                 targets.setdefault(proj.target, []).append(proj)
         if not targets:
-            return ""
+            return "", ""
+        # (four neurons per thread: too many registers)
+        early = K <= 2 and sum(len(v) for v in targets.values()) <= 4
+        held, first, second = [], [], []
 
-        def value(name, src):
-            return f"anb_h_{name}[anb_k]" if K > 1 else f"{src}[anb_i]"
+        # (before the inboxes: their chain of loads would hold back the state's)
+        def value(name):
+            return f"anb_h_{name}[anb_k]"
 
         decl, fetch, work, clear = [], [], [], []
         for T, projs in targets.items():
@@ -712,13 +723,13 @@ class CodeGenerator:
                 loads[loads.index(f"{R} g_{T} = {src}[anb_i];")] = f"{R} g_{T} = anb_gd_{T};"
             hoist.append((R, f"anb_in_g_{T}", src))
             decl.append(f"{R} anb_gd_{T} = ({R})0;")
-            fetch.append(f"anb_gd_{T} = {value(f'anb_in_g_{T}', src)};")
+            fetch.append(f"anb_gd_{T} = {value(f'anb_in_g_{T}')};")
             for proj in projs:
                 k = proj.id
                 p = lambda n: self.ptr(f"proj{k}__{n}")
                 hoist.append(("anb_u32", f"anb_in_c{k}", p("ibn")))
                 decl.append(f"anb_u32 anb_ic{k} = 0u;")
-                fetch.append(f"anb_ic{k} = {value(f'anb_in_c{k}', p('ibn'))};")
+                fetch.append(f"anb_ic{k} = {value(f'anb_in_c{k}')};")
                 w = p("pv") if proj.plastic else p("w")
                 rows = f"{p('row_ptr')}[anb_r], {p('row_ptr')}[anb_r + 1], {p('col')}, {w}"
                 if proj._delay_steps is not None:
@@ -728,7 +739,24 @@ class CodeGenerator:
                             f"{self.slots(a)}, t)")
                 else:
                     walk = f"anb_row_gather<{R}>(anb_g, {rows}, {p('ibb')})"
-                work.append(f"""
+                short = ""
+                if early:
+                    key = "unsigned long long" if proj._delay_steps is not None else "anb_u32"
+                    c = f"anb_h_anb_in_c{k}[anb_k]"
+                    held.append(f"{key} anb_ea{k}[{K}], anb_eb{k}[{K}]; {R} anb_va{k}[{K}], anb_vb{k}[{K}];")
+                    # (one neuron per thread: without waiting for the counts)
+                    first.append(f"{'' if K == 1 else f'if ({c}) '}"
+                                 f"anb_inbox_first({p('ibx')}, anb_j, anb_ea{k}[anb_k], anb_eb{k}[anb_k]);")
+                    second.append(f"anb_va{k}[anb_k] = {c} == 1u || {c} == 2u ? {w}[(anb_u32)anb_ea{k}[anb_k]] : ({R})0; "
+                                  f"anb_vb{k}[anb_k] = {c} == 2u ? {w}[(anb_u32)anb_eb{k}[anb_k]] : ({R})0;")
+                    short = f"""
+          if (anb_ic{k} == 1u || anb_ic{k} == 2u) {{
+            // (ascending keys: the reference's order of additions)
+            const bool anb_o = anb_ic{k} == 2u && anb_eb{k}[anb_k] < anb_ea{k}[anb_k];
+            anb_gd_{T} += anb_o ? anb_vb{k}[anb_k] : anb_va{k}[anb_k];
+            if (anb_ic{k} == 2u) anb_gd_{T} += anb_o ? anb_va{k}[anb_k] : anb_vb{k}[anb_k];
+          }} else"""
+                work.append(f"""{short}
           if (anb_ic{k} && anb_ic{k} <= ANB_INBOX)
             anb_gd_{T} = anb_inbox_add(anb_gd_{T}, anb_ic{k}, {p('ibx')}, anb_i, {w});
           for (anb_u32 anb_m = __ballot_sync(0xffffffffu, anb_ic{k} > ANB_INBOX); anb_m; anb_m &= anb_m - 1) {{
@@ -751,6 +779,20 @@ class CodeGenerator:
         }}
         if (__any_sync(0xffffffffu, ({any_}) != 0u)) {{{''.join(work)}
           {nl.join(clear)}
+        }}""", "" if not early else f"""
+        {nl.join(held)}
+#pragma unroll
+        for (int anb_k = 0; anb_k < {K}; ++anb_k) {{
+          const int anb_j = anb_base0 + anb_k * blockDim.x + threadIdx.x;
+          if (anb_j < anb_n) {{
+          {nl.join(first)}
+          }}
+        }}
+#pragma unroll
+        for (int anb_k = 0; anb_k < {K}; ++anb_k) {{
+          if (anb_base0 + anb_k * blockDim.x + threadIdx.x < anb_n) {{
+          {nl.join(second)}
+          }}
         }}"""
 
     @staticmethod
@@ -783,11 +825,21 @@ class CodeGenerator:
       }}
     }}"""
         dt_t = "double" if self.exact else "float"
+        # (population-level variables are written every step)
+        before, after = ("", preamble) if geq or pop._globalops else (preamble, "")
+        events = self._post_constants(pop)
+        if any(v["locality"] == "global" for p in self.net.projections
+               if p.post_pop is pop and self.post_fused(p) for v in p.desc["variables"]):
+            after += "\n    " + events
+        else:
+            before += "\n    " + events
         return f"""
 extern "C" __global__ void __launch_bounds__({BLOCK}) pop{k}_step() {{
-    const long long t = *{self.ptr('t')};
     const {dt_t} dt = ({dt_t})(*{self.ptr('dt')});
-    {preamble}
+    {before}
+    {ENTER}
+    const long long t = *{self.ptr('t')};
+    {after}
 {self.neuron_update(pop)}{store}
 }}
 """
@@ -1659,12 +1711,15 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) proj{k}_psp() {{
         # fast: work items (spike of the previous step, 32-synapse chunk of its
         # fan-out); the synapse state is reached through inv_idx
         a = proj.pre_pop.id
+        known = "\n    ".join(f"const {ct} {n} = {src}[0];" for ct, n, src in self._constants(proj))
+        written = any(v["locality"] == "global" for v in proj.desc["variables"])
         return f"""
 extern "C" __global__ void __launch_bounds__({BLOCK}) proj{k}_psp() {{
-    const long long t = *{self.ptr('t')};
     const float dt = (float)(*{self.ptr('dt')});
-    const int anb_plastic = {p('flags')}[0];
-    {self._syn_globals(proj)}
+    {"" if written else known}
+    {ENTER}
+    const long long t = *{self.ptr('t')};
+    {known if written else ""}
     {self._syn_arrays(proj)}
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1717,12 +1772,28 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) proj{k}_psp() {{
             if delay:
                 put = f"if ({delay}) {put}"
             decl = ""
+            now = f"""{ENTER}
+      const long long t = *{self.ptr('t')};"""
+            find = f"""const int anb_ns = anb_list_spikes(anb_list, {bits} + {lay['w0']}, {(a.size + 31) // 32}, {lay['w0']}, {words}, {slots}, t,
+                                         anb_w, anb_nw, {p('col_ptr')}, nullptr);"""
+            if not slots and per * 32 <= BLOCK:
+                # a thread per neuron: the column's bounds before the wait
+                now = f"""const int anb_id = ({lay['w0']} + anb_w) * 32 + (int)threadIdx.x;
+      const bool anb_in = (int)threadIdx.x < anb_nw * 32 && anb_id < {a.size};
+      const int anb_pb = anb_in ? {p('col_ptr')}[anb_id] : 0, anb_pe = anb_in ? {p('col_ptr')}[anb_id + 1] : 0;
+      {now}"""
+                find = f"""const anb_u32* anb_bits = {bits};
+      const int anb_ns = anb_list_ranges(anb_list, ((int)threadIdx.x & 31) < anb_nw ? anb_bits[{lay['w0']} + anb_w + (threadIdx.x & 31)] : 0u,
+                                         anb_id, anb_pb, anb_pe);"""
             if proj.plastic:
                 stmts = self._event_driven(proj, "j", "t-1") + self.syn_spike_statements(proj, "pre_spike")
                 body = "\n          ".join(stmts)
-                decl = f"""const int anb_plastic = {p('flags')}[0];
-      {self._syn_globals(proj)}
-      {self._syn_arrays(proj)}"""
+                decl = self._syn_arrays(proj)
+                known = "\n      ".join(f"const {ct} {n} = {src}[0];" for ct, n, src in self._constants(proj))
+                if any(v["locality"] == "global" for v in proj.desc["variables"]):
+                    now += "\n      " + known
+                else:
+                    decl += "\n      " + known
                 put = f"""const int j = anb_j;
           {self.real} sum = ({self.real})0;
           {self.syn_index_defs(body, "anb_pre", f"{p('post_idx')}[anb_q]")}{body}
@@ -1733,13 +1804,13 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) proj{k}_psp() {{
       const int anb_w = ((int)blockIdx.x - {first}) * {per};
       const int anb_nw = min({per}, {words * max(1, slots)} - anb_w);
       {decl}
+      {now}
       const anb_u32* anb_old = {oldest};
       for (int q = (int)blockIdx.x - {first}; q < {-(-words // BLOCK)}; q += {ctas}) {{
         const int anb_cw = q * {BLOCK} + threadIdx.x;
         if (anb_cw < {words}) {p('ibb')}[{lay['w0']} + anb_cw] = anb_old[{lay['w0']} + anb_cw];
       }}
-      const int anb_ns = anb_list_spikes(anb_list, {bits} + {lay['w0']}, {(a.size + 31) // 32}, {lay['w0']}, {words}, {slots}, t,
-                                         anb_w, anb_nw, {p('col_ptr')}, nullptr);
+      {find}
       anb_for_spikes(anb_list, anb_ns, [&](const int anb_pre, const int anb_d, const int anb_q) {{
           const int anb_j = {p('inv_idx')}[anb_q];
           {put}
@@ -1749,7 +1820,6 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) proj{k}_psp() {{
         name = "anb_deliver"
         return f"""
 extern "C" __global__ void __launch_bounds__({BLOCK}) {name}() {{
-    const long long t = *{self.ptr('t')};
     const {self.real} dt = ({self.real})(*{self.ptr('dt')});
     __shared__ int anb_list[4 * ANB_DELIVER_LIST + 1];
     {''.join(parts)}
@@ -1763,7 +1833,8 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) {name}() {{
         fork and a join per step and the launches before and after them could
         not overlap (programmatic dependent launch follows one stream): with
         the post events in the update kernel, 20,000 neurons with 1.3M plastic
-        synapses took 10.1 us per step that way and take 7.5 us."""
+        synapses took 10.1 us per step that way, 7.5 in one launch (and 6.1 with
+        the single values read before the wait for the previous kernel)."""
         parts, first = [], 0
         for proj in projs:
             n = self.c.layout[proj.id]["grid"]
@@ -1771,6 +1842,8 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) {name}() {{
             body = src[src.index("{") + 1:src.rindex("}")]
             body = body.replace("(int)blockIdx.x", "anb_blk").replace("(int)gridDim.x", "anb_nblk")
             body = body.replace("blockIdx.x", "anb_blk").replace("gridDim.x", "anb_nblk")
+            if ENTER not in body:              # (every CTA runs one of the parts)
+                body = f"\n    {ENTER}" + body
             parts.append(f"""
     if ((int)blockIdx.x >= {first} && (int)blockIdx.x < {first + n}) {{  // {proj.name}
       const int anb_blk = (int)blockIdx.x - {first}, anb_nblk = {n};{body.rstrip()}
@@ -1847,13 +1920,19 @@ __device__ __noinline__ anb_tr{k} proj{k}_post_syn(anb_tr{k} anb_s, const long l
         parts = []
         for proj in projs:
             p = lambda n, k=proj.id: self.ptr(f"proj{k}__{n}")
+            k = proj.id
+            known = "\n          ".join(f"const {ct} {n} = anb_c{k}_{n};" for ct, n, _ in self._constants(proj))
+            find = f"""const int anb_ns = anb_list_spikes(anb_list, anb_sw, 0, anb_first / 32, {words}, 0, t, 0, {words},
+                                             {p('row_ptr')}, {p('row_of')});"""
+            if K == 1:
+                # (a population with one neuron per thread is one pass of the grid)
+                find = f"""const int anb_ns = anb_list_ranges(anb_list, (threadIdx.x & 31) < {words} ? anb_sw[threadIdx.x & 31] : 0u,
+                                             anb_i0, anb_rb{k}, anb_re{k});"""
             parts.append(f"""
         {{  // {proj.name}
-          const int anb_plastic = {p('flags')}[0];
-          {self._syn_globals(proj)}
+          {known}
           {self._syn_arrays(proj)}
-          const int anb_ns = anb_list_spikes(anb_list, anb_sw, 0, anb_first / 32, {words}, 0, t, 0, {words},
-                                             {p('row_ptr')}, {p('row_of')});
+          {find}
           anb_for_spikes(anb_list, anb_ns, [&](const int anb_post, const int anb_d, const int j) {{
             {self._post_body(proj)}
           }});
@@ -1862,6 +1941,38 @@ __device__ __noinline__ anb_tr{k} proj{k}_post_syn(anb_tr{k} anb_s, const long l
         return keep, f"""
         if (__syncthreads_or(anb_any != 0u)) {{{''.join(parts)}
         }}"""
+
+    def _constants(self, proj) -> list:
+        """(type, name, array) of a plastic projection's single values."""
+        p = lambda n: self.ptr(f"proj{proj.id}__{n}")
+        return [("int", "anb_plastic", p("flags"))] + [
+            (self.real, prm["name"], p(prm["name"])) for prm in proj.desc["parameters"] + proj.desc["variables"]
+            if prm["locality"] == "global"]
+
+    def _post_constants(self, pop) -> str:
+        """What the post events of the update kernel read and no kernel
+        writes: single values, and the thread's row of synapses (were two
+        dependent loads after the spike: row number, then its bounds)."""
+        out = []
+        n = pop.size
+        first = 0
+        if pop.id in getattr(self.c, "owned", {}):
+            first, n = self.c.owned[pop.id]
+        projs = [p for p in self.net.projections if p.post_pop is pop and self.post_fused(p)]
+        rows = projs and self.neurons_per_thread(pop) == 1
+        if rows:
+            out.append(f"const int anb_i0 = {first} + blockIdx.x * blockDim.x + threadIdx.x;")
+        for proj in projs:
+            k = proj.id
+            p = lambda n, k=k: self.ptr(f"proj{k}__{n}")
+            out += [f"const {ct} anb_c{k}_{nm} = {src}[0];" for ct, nm, src in self._constants(proj)]
+            if rows:
+                out.append(f"""int anb_rb{k} = 0, anb_re{k} = 0;
+    {{
+      const int anb_r = anb_i0 < {n} ? {p('row_of')}[anb_i0] : -1;
+      if (anb_r >= 0) {{ anb_rb{k} = {p('row_ptr')}[anb_r]; anb_re{k} = {p('row_ptr')}[anb_r + 1]; }}
+    }}""")
+        return "\n    ".join(out)
 
     def post_event_kernel(self, proj) -> str:
         k = proj.id
@@ -2173,8 +2284,7 @@ extern "C" __global__ void __launch_bounds__({PERSISTENT_BLOCK}, 1) anb_grid_run
                 stops.append((pop.id, f"pop{pop.id}_stop", grid_for(pop.size), BLOCK, mode_all))
         # every kernel first waits for its predecessor on the stream (the plan
         # is launched with programmatic dependent launch)
-        kernels = [re.sub(r'(extern "C" __global__ void (?:__launch_bounds__\([^)]*\) )?\w+\(\) \{)',
-                          r"\1\n    anb_pdl_enter();", src) for src in kernels]
+        kernels = [self._at_entry(src, r"\w+", "\n    anb_pdl_enter();").replace(ENTER, "") for src in kernels]
         # several kernels: compiled in parallel (a plastic double-precision
         # module 354 -> 240 ms on 8 cores; a single kernel gains nothing)
         return Module(self.assemble(kernels), self.options() + ["--split-compile=0"], "grid", plan=plan,
@@ -2210,9 +2320,22 @@ extern "C" __global__ void anb_tick() {
 
     @staticmethod
     def _prologue(kernels: list, name: str, code: str) -> list:
-        """Insert `code` after the opening brace of kernel `name`."""
-        return [re.sub(rf'(extern "C" __global__ void (?:__launch_bounds__\([^)]*\) )?{name}\(\) \{{)',
-                       lambda m: m.group(1) + code, src) for src in kernels]
+        """Insert `code` at the entry of kernel `name`."""
+        return [CodeGenerator._at_entry(src, name, code) for src in kernels]
+
+    @staticmethod
+    def _at_entry(src: str, name: str, code: str) -> str:
+        """Insert `code` where the kernels matching `name` wait for their
+        predecessor: at the marks of their source (ENTER), else after the
+        opening brace."""
+        head = re.compile(rf'extern "C" __global__ void (?:__launch_bounds__\([^)]*\) )?{name}\(\) \{{')
+        parts = re.split(r'(?=extern "C" __global__ void )', src)
+        for i, part in enumerate(parts):
+            m = head.match(part)
+            if m:
+                parts[i] = (part.replace(ENTER, ENTER + code) if ENTER in part
+                            else part[:m.end()] + code + part[m.end():])
+        return "".join(parts)
 
     @staticmethod
     def _append_epilogue(kernels: list, name: str, code: str) -> list:
