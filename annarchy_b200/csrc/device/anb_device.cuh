@@ -981,7 +981,12 @@ __device__ __forceinline__ void anb_spike_gather_delayed(int n_rows, const int* 
 // atomics. Measured per step against the row-walking kernels: 100,000 neurons
 // with 500 synapses each 139 -> 15.5 us, 10,000 neurons with 0.8M plastic
 // synapses 22.8 -> 11.8 us, 3000 neurons with a delay per synapse 10.2 -> 8.3
-// us (the last two are the launches and the chains of dependent loads).
+// us (the last two are the launches and the chains of dependent loads). With
+// what no kernel writes loaded before the wait for the previous kernel, and the
+// bounds of a word's columns by a thread per neuron, the first two 13.8 and 9.6
+// us; with the entries of all inboxes of a thread fetched at once, 11.4 and 9.6;
+// with a plastic synapse's place in the inbox asked for before its statements,
+// 8.4 for the plastic one.
 #define ANB_INBOX 8          // entries per post neuron: one 32-byte sector of 32-bit keys
 #define ANB_DELIVER_WORDS 32 // bitmap words per CTA of a deliver kernel, at most
 #define ANB_DELIVER_LIST (32 * ANB_DELIVER_WORDS)

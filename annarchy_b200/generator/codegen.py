@@ -1733,10 +1733,10 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) proj{k}_psp() {{
       const int anb_end = {p('col_ptr')}[anb_pre + 1];
       for (int anb_k = {p('col_ptr')}[anb_pre] + anb_c * 32 + lane; anb_k < anb_end;
            anb_k += 32 * {lay['chunks']}) {{
-        const int j = {p('inv_idx')}[anb_k];
+        const int j = {p('inv_idx')}[anb_k], anb_po = {p('post_idx')}[anb_k];
         float sum = 0.f;
-        {self.syn_index_defs(body, "anb_pre", f"{p('post_idx')}[anb_k]")}{body}
-        atomicAdd(&{g}[{p('post_idx')}[anb_k]], sum);
+        {self.syn_index_defs(body, "anb_pre", "anb_po")}{body}
+        atomicAdd(&{g}[anb_po], sum);
       }}
     }}
 }}
@@ -1794,11 +1794,16 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) proj{k}_psp() {{
                     now += "\n      " + known
                 else:
                     decl += "\n      " + known
+                # the place in the inbox is asked for before the statements: its
+                # trip to L2 and theirs overlap (a delay's step decides first)
+                enter = f"""const int anb_po = {p('post_idx')}[anb_q];
+          const anb_u32 anb_place = {f'!({delay}) ? ANB_INBOX : ' if delay else ''}atomicAdd(&{p('ibn')}[anb_po], 1u);"""
                 put = f"""const int j = anb_j;
+          {enter}
           {self.real} sum = ({self.real})0;
-          {self.syn_index_defs(body, "anb_pre", f"{p('post_idx')}[anb_q]")}{body}
+          {self.syn_index_defs(body, "anb_pre", "anb_po")}{body}
           {p('pv')}[j] = sum;
-          {put}"""
+          if (anb_place < ANB_INBOX) {p('ibx')}[(size_t)anb_po * ANB_INBOX + anb_place] = {key};"""
             parts.append(f"""
     if ((int)blockIdx.x >= {first} && (int)blockIdx.x < {first + ctas}) {{  // {proj.name}
       const int anb_w = ((int)blockIdx.x - {first}) * {per};
