@@ -196,7 +196,20 @@ class Batch:
         for name in compensated_vars(pop, self.exact, self.comp_config(pop)):
             out.append(("kc_" + name, "float"))
         out.append(("spk", "anb_u32"))
+        if self.counted:
+            # events of the step per neuron and projection
+            out += [(f"cnt{pr.id}", "short") for pr in self.net.projections if pr.post_pop is pop]
         return out
+
+    def _one_weight(self) -> bool:
+        """Every projection of every instance carries one weight, and no
+        neuron can get 65536 events in a step."""
+        for n in self.networks:
+            for pr in n.projections:
+                w = pr._csr.data
+                if (w.size and not np.all(w == w[0])) or pr.pre_pop.size >= 65536:
+                    return False
+        return True
 
     def comp_config(self, pop) -> dict:
         if self.compensate != "auto":
@@ -222,6 +235,8 @@ class Batch:
         for proj in self.net.projections:
             k = proj.id
             longs.append((f"cp{k}", f"proj{k}__bcpoff", 1, 0))
+            if self.counted:
+                reals.append((f"w{k}", f"proj{k}__bw", 1, 0))
             ints += [(f"wr{k}_0", f"proj{k}__bwr", 2, 0), (f"wr{k}_1", f"proj{k}__bwr", 2, 1)]
         ints += [(f"so{c}", "bt__soff", self.n_arrays, c) for c in range(self.n_arrays)]
         rs = 8 if self.exact else 4
@@ -278,36 +293,16 @@ class Batch:
         nets = self.networks
         nat = self.native
         nat.initialize(self.net.dt)
-        self.smem_arrays = {p.id: self._smem_arrays(p) for p in self.net.populations}
-        self.array_index = {}
-        for pop in self.net.populations:
-            for name, _ in self.smem_arrays[pop.id]:
-                self.array_index[(pop.id, name)] = len(self.array_index)
-        self.n_arrays = len(self.array_index)
-        inst = [self._instance_bytes(n) for n in nets]
-        # every instance also takes one header slot at the start of its CTA's
-        # shared memory
-        self.header_bytes = self.header_layout()[3]
-        sizes = [b + self.header_bytes for _, b in inst]
-        # synapse indices in 32 bits while every projection's concatenation fits
-        tot = max([sum(n.projections[j].nb_synapses for n in nets)
-                   for j in range(len(self.net.projections))] or [0])
-        self.idx_t = "int" if tot + 8 < 2**31 - 1 else "long long"
-        # fast mode keeps room for the delivery scratch: 32 warp sums, the
-        # list counter, then at least 512 list entries, each with its
-        # synapse range in every projection
-        isz = 4 if self.idx_t == "int" else 8
-        self.entry_bytes = 4 + 2 * isz * len(self.net.projections)
-        limit = SMEM_LIMIT - (0 if self.exact else 4 * 36 + 512 * self.entry_bytes + 16)
-        if max(sizes) > limit:
-            i = int(np.argmax(sizes))
-            raise ValueError(f"instance {i} needs {sizes[i]} bytes of shared memory "
-                             f"(at most {limit} per CTA in this precision)")
-        nnz = [sum(pr.nb_synapses for pr in n.projections) for n in nets]
-        neurons = [sum(p.size for p in n.populations) for n in nets]
-        costs = [neurons[i] + 0.01 * nnz[i] for i in range(len(nets))]
-        sms = self.ctas or (148 if self.dry else device_sm_count(self.device))
-        where, n_cta = self._pack(costs, sizes, min(len(nets), sms), limit)
+        # double precision with one weight per projection: events are counted,
+        # unless the counters would need more waves of CTAs. 96 instances of
+        # 400 to 2800 neurons: 16.8 -> 7.2 us per step, 24 of 600 to 1800: 7.7
+        # -> 5.4. (Single precision keeps adding weights with atomics: 5.7 and
+        # 4.4 us, 5.9 and 4.5 with counters.)
+        plans = [True, False] if self.exact and self._one_weight() else [False]
+        for self.counted in plans:
+            where, n_cta, sizes, inst, costs = self._plan()
+            if where is not None:
+                break
         # slots: instances in CTA order
         order = np.lexsort((np.arange(len(nets)), where))
         self.order = order                      # slot -> instance
@@ -335,9 +330,10 @@ class Batch:
         # with a list of list_cap entries (a multiple of 4)
         self.smem_state = -(-int(max(np.bincount(where, weights=sizes, minlength=n_cta))) // 16) * 16
         free = SMEM_LIMIT - self.smem_state - 4 * 36
-        self.list_cap = 0 if self.exact else int(min(1024, free // self.entry_bytes) // 4 * 4)
-        assert self.exact or self.list_cap >= 512
-        self.smem = self.smem_state + (0 if self.exact else 4 * 36 + self.list_cap * self.entry_bytes)
+        listed = self.counted or not self.exact
+        self.list_cap = int(min(1024, free // self.entry_bytes) // 4 * 4) if listed else 0
+        assert not listed or self.list_cap >= 512
+        self.smem = self.smem_state + (0 if not listed else 4 * 36 + self.list_cap * self.entry_bytes)
         words = np.array([sum((p.size + 31) // 32 for p in n.populations) for n in nets])
         cta_words = np.bincount(where, weights=words, minlength=n_cta)
         if cta_words.max() > 1024:
@@ -354,6 +350,46 @@ class Batch:
             n._compiled = True
         self.compiled = True
         return self
+
+    def _plan(self):
+        """Shared-memory layout and packing: CTA of every instance (None:
+        does not fit with event counters), CTAs, bytes, offsets and costs."""
+        nets = self.networks
+        self.smem_arrays = {p.id: self._smem_arrays(p) for p in self.net.populations}
+        self.array_index = {}
+        for pop in self.net.populations:
+            for name, _ in self.smem_arrays[pop.id]:
+                self.array_index[(pop.id, name)] = len(self.array_index)
+        self.n_arrays = len(self.array_index)
+        inst = [self._instance_bytes(n) for n in nets]
+        # every instance also takes one header slot at the start of its CTA's
+        # shared memory
+        self.header_bytes = self.header_layout()[3]
+        sizes = [b + self.header_bytes for _, b in inst]
+        # synapse indices in 32 bits while every projection's concatenation fits
+        tot = max([sum(n.projections[j].nb_synapses for n in nets)
+                   for j in range(len(self.net.projections))] or [0])
+        self.idx_t = "int" if tot + 8 < 2**31 - 1 else "long long"
+        # fast mode keeps room for the delivery scratch: 32 warp sums, the
+        # list counter, then at least 512 list entries, each with its
+        # synapse range in every projection
+        isz = 4 if self.idx_t == "int" else 8
+        self.entry_bytes = 4 + 2 * isz * len(self.net.projections)
+        limit = SMEM_LIMIT - (0 if self.exact and not self.counted else 4 * 36 + 512 * self.entry_bytes + 16)
+        if self.counted and max(sizes) > limit:
+            return None, 0, sizes, inst, None
+        if max(sizes) > limit:
+            i = int(np.argmax(sizes))
+            raise ValueError(f"instance {i} needs {sizes[i]} bytes of shared memory "
+                             f"(at most {limit} per CTA in this precision)")
+        nnz = [sum(pr.nb_synapses for pr in n.projections) for n in nets]
+        neurons = [sum(p.size for p in n.populations) for n in nets]
+        costs = [neurons[i] + 0.01 * nnz[i] for i in range(len(nets))]
+        sms = self.ctas or (148 if self.dry else device_sm_count(self.device))
+        where, n_cta = self._pack(costs, sizes, min(len(nets), sms), limit)
+        if self.counted and n_cta > min(len(nets), sms):
+            return None, 0, sizes, inst, None
+        return where, n_cta, sizes, inst, costs
 
     def _create_populations(self, order):
         nat = self.native
@@ -441,6 +477,8 @@ class Batch:
                 post, w = post[perm], w[perm]
             # the fast delivery reads aligned groups of 4 synapses: pad the
             # arrays so that the last group stays inside them
+            if self.counted:
+                nat.create(f"proj{k}__bw", np.array([x[0] if x.size else 0.0 for x in ws], dtype=self.real))
             pad = (-post.size) % 4 + 4
             post = np.concatenate([post, np.zeros(pad, np.int64)])
             w = np.concatenate([w, np.zeros(pad)])

@@ -1359,6 +1359,17 @@ __device__ __forceinline__ R anb_mask_drain(R g, R w, unsigned short* cnt) {
     if (c > 0) g += w;
   return g;
 }
+// The same without votes (lanes on their own).
+template <typename R>
+__device__ __forceinline__ R anb_count_add(R g, R w, unsigned short* cnt) {
+  int c = *cnt;
+  if (c) {
+    *cnt = 0;
+    do g += w;
+    while (--c);
+  }
+  return g;
+}
 // Store of one word into another CTA of the cluster, counted on that CTA's
 // mbarrier (launches with a cluster only; the own CTA's word is an ordinary
 // store).

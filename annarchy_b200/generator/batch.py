@@ -10,8 +10,11 @@ Instances never exchange data, so the only barriers are the CTA's own:
 
     for every step:
         deliver the spikes of the previous step of every own instance
-        (fast: shared-memory atomics; exact: spike by spike in ascending pre
-        rank with one CTA barrier per spike, the reference's per-post order)
+        (fast: shared-memory atomics; exact: where every projection has one
+        weight, events counted per neuron and projection by shared-memory
+        atomics and the weight added as often by the update, else spike by
+        spike in ascending pre rank with one CTA barrier per spike, the
+        reference's per-post order)
         __syncthreads
         update every own instance's neurons, spike bitmap words by ballot
         (and into the spike monitor ring)
@@ -117,6 +120,10 @@ class BatchGenerator(CodeGenerator):
         lines, d = self._smem_ptrs(pop)
         body = []
         for name, ct in self.b.smem_arrays[k]:
+            if name.startswith("cnt"):        # (none left over between launches)
+                if to_smem:
+                    body.append(f"for (int q = threadIdx.x; q < anb_n{k}; q += blockDim.x) {d[name]}[q] = 0;")
+                continue
             if name == "spk":
                 g = f"{self.ptr(f'pop{k}__spk')}[anb_woff{k} + q]"
                 n = f"((anb_n{k} + 31) >> 5)"
@@ -193,7 +200,7 @@ class BatchGenerator(CodeGenerator):
         synapse range in every projection leaving the population (the column
         pointers are read here, where their latency hides behind the other
         warps' updates), and the range's synapse words are prefetched into L2."""
-        if self.exact or pop not in spk_pops:
+        if (self.exact and not self.b.counted) or pop not in spk_pops:
             return ""
         pi = spk_pops.index(pop)
         P = len(spk_pops)
@@ -210,7 +217,8 @@ class BatchGenerator(CodeGenerator):
             else:
                 pref = [(self.ptr(f"proj{k}__post"), 4)]
                 wsize = {np.float64: 8, np.float32: 4}.get(self.b.wdtype, 2)
-                pref.append((self.ptr(f"proj{k}__w"), wsize))
+                if not self.b.counted:
+                    pref.append((self.ptr(f"proj{k}__w"), wsize))
             pf = []
             for arr, size in pref:
                 # aligned to 16 bytes on both ends; the arrays are padded so
@@ -273,8 +281,16 @@ class BatchGenerator(CodeGenerator):
             pi = spk_pops.index(proj.pre_pop)
             k = proj.id
             g_col = self.b.array_index[(proj.post_pop.id, "g_" + proj.target)]
-            U = 4 if self.b.packed.get(k) else 2
-            if self.b.packed.get(k):
+            U = 4 if self.b.packed.get(k) or self.b.counted else 2
+            if self.b.counted:
+                # (two counters of 16 bits in a word)
+                g_col = self.b.array_index[(proj.post_pop.id, f"cnt{k}")]
+                load = (f"anb_p4[u] = anb_ls_i4(reinterpret_cast<const int4*>({self.ptr(f'proj{k}__post')}) + anb_g);")
+                regs = "int4 anb_p4[4];"
+                add = "ANB_ADD(anb_p4[u].x, 0) ANB_ADD(anb_p4[u].y, 1) ANB_ADD(anb_p4[u].z, 2) ANB_ADD(anb_p4[u].w, 3)"
+                macro = ("#define ANB_ADD(po, c) if (anb_g * 4 + c >= anb_bq[u] && anb_g * 4 + c < anb_eq[u]) "
+                         "atomicAdd(reinterpret_cast<anb_u32*>(anb_smem + anb_go[u]) + ((po) >> 1), ((po) & 1) ? 0x10000u : 1u);")
+            elif self.b.packed.get(k):
                 syn = self.ptr(f"proj{k}__syn")
                 load = f"anb_v[u] = anb_ls_u4(reinterpret_cast<const uint4*>({syn}) + anb_g);"
                 regs = "uint4 anb_v[4];"
@@ -428,6 +444,16 @@ class BatchGenerator(CodeGenerator):
         upd = self.neuron_update(pop, local_engine=True, smem=d, ballot_hook=hook,
                                  size=f"anb_n{k}", gsrc=self._pop_gsrc(k), refractory=refr)
         nl = "\n        "
+        if self.b.counted:
+            # the step's events, projection by projection: the weight as often
+            # as counted is the reference's sequence of additions
+            for target in {pr.target for pr in self.net.projections if pr.post_pop is pop}:
+                load = f"{self.real} g_{target} = {d['g_' + target]}[anb_i];"
+                assert upd.count(load) == 1, load
+                upd = upd.replace(load, load + "".join(
+                    f" g_{target} = anb_count_add(g_{target}, {self._hx(f'w{pr.id}')}, "
+                    f"reinterpret_cast<unsigned short*>({d[f'cnt{pr.id}']}) + anb_i);"
+                    for pr in self.net.projections if pr.post_pop is pop and pr.target == target))
         return f"""
       {{
         {nl.join(lines)}
@@ -450,7 +476,7 @@ class BatchGenerator(CodeGenerator):
         load = "".join(self._copy(p, True) for p in pops)
         store = "".join(self._copy(p, False) for p in pops)
         spk_pops = self._spk_pops()
-        if self.exact:
+        if self.exact and not self.b.counted:
             deliver = (f"for (int anb_si = anb_sb; anb_si < anb_se; ++anb_si) {{\n        {header}"
                        + "".join(self._delivery_exact(pr) for pr in net.projections) + "\n      }")
         elif spk_pops:
@@ -459,7 +485,7 @@ class BatchGenerator(CodeGenerator):
             deliver = ""
         update = "".join(self._update(p) for p in pops)
         dt_t = "double" if self.exact else "float"
-        scratch = "" if self.exact or not spk_pops else self._scratch(spk_pops)
+        scratch = "" if (self.exact and not self.b.counted) or not spk_pops else self._scratch(spk_pops)
         if scratch:
             # no list at the first step of a launch: the delivery rebuilds it
             # from the spike bitmaps
