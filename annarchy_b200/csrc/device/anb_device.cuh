@@ -390,8 +390,9 @@ __device__ __forceinline__ float anb_w1(const anb_bf16* w) { return anb_bf16_to_
 // Sub-warp per row with 16-byte vector loads of the column indices and
 // weights (streaming, evict-first) over the 4-aligned body of every row and
 // scalar loads at its ends. `rows` (optional) lists the rows to process
-// (row-length binning); `n_rows` is its length.
-template <int G, typename W>
+// (row-length binning); `n_rows` is its length. ATOMIC: other sums are added to
+// the same neurons meanwhile.
+template <int G, typename W, bool ATOMIC = false>
 __device__ __forceinline__ void anb_rate_csr_vec(int n_rows, const int* __restrict__ rows,
                                                  const int* __restrict__ row_ptr,
                                                  const int* __restrict__ col,
@@ -401,9 +402,11 @@ __device__ __forceinline__ void anb_rate_csr_vec(int n_rows, const int* __restri
                                                  float* __restrict__ sum) {
   const int lane = threadIdx.x % G;
   const int groups = (gridDim.x * blockDim.x) / G;
-  for (int r = (blockIdx.x * blockDim.x + threadIdx.x) / G; r < n_rows; r += groups) {
-    const int row = rows ? rows[r] : r;
-    const int beg = row_ptr[row], end = row_ptr[row + 1];
+  // (a warp's lanes stay together: all of them take part in the shuffles)
+  const int in_warp = (threadIdx.x & 31) / G;
+  for (int r = (blockIdx.x * blockDim.x + threadIdx.x) / G; r - in_warp < n_rows; r += groups) {
+    const int row = r >= n_rows ? -1 : rows ? rows[r] : r;
+    const int beg = row < 0 ? 0 : row_ptr[row], end = row < 0 ? 0 : row_ptr[row + 1];
     int j0 = (beg + 3) & ~3;
     if (j0 > end) j0 = end;
     float s = 0.f;
@@ -430,7 +433,13 @@ __device__ __forceinline__ void anb_rate_csr_vec(int n_rows, const int* __restri
     for (int j = j0 + 4 * nv + lane; j < end; j += G) s += __ldg(&x[anb_ls_i(&col[j])]) * anb_w1(&w[j]);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, G);
-    if (lane == 0) sum[post_rank ? post_rank[row] : row] += s;
+    if (lane == 0 && row >= 0) {
+      float* const to = &sum[post_rank ? post_rank[row] : row];
+      if (ATOMIC)
+        atomicAdd(to, s);
+      else
+        *to += s;
+    }
   }
 }
 
@@ -762,13 +771,17 @@ __device__ __forceinline__ float anb_pc_w(const anb_bf16* w) {
   return __uint_as_float((unsigned)__ldcs(reinterpret_cast<const unsigned short*>(w)) << 16);
 }
 
-template <typename W, int U>
+//
+// wait(): called once, after what the step does not change (the work split and
+// the first entries) has been asked for and before x is read.
+template <typename W, int U, typename Wait>
 __device__ __forceinline__ void anb_rate_pcsr(const int* __restrict__ cta_panel,
                                               const int* __restrict__ warp_tab,
                                               const unsigned short* __restrict__ col,
                                               const W* __restrict__ w,
                                               const float* __restrict__ x, int n_pre,
-                                              int panel_width, float* __restrict__ sum, int* err) {
+                                              int panel_width, float* __restrict__ sum, int* err,
+                                              Wait&& wait) {
   extern __shared__ __align__(16) unsigned char anb_pc_smem[];
   __shared__ __align__(8) unsigned long long anb_pc_mbar;
   float* xs = reinterpret_cast<float*>(anb_pc_smem);
@@ -776,8 +789,6 @@ __device__ __forceinline__ void anb_rate_pcsr(const int* __restrict__ cta_panel,
   const int c0 = p * panel_width;
   const int cw = min(panel_width, n_pre - c0);
   const int cw4 = cw & ~3;
-  if (threadIdx.x == 0 && cw4 > 0) anb_bulk_issue(xs, x + c0, 4u * (unsigned)cw4, &anb_pc_mbar);
-  for (int q = cw4 + threadIdx.x; q < cw; q += blockDim.x) xs[q] = x[c0 + q];
   const int lane = threadIdx.x & 31;
   const int* wt = warp_tab + 3 * (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
   const int sb = wt[0], se = wt[1], hd = wt[2];
@@ -824,6 +835,9 @@ __device__ __forceinline__ void anb_rate_pcsr(const int* __restrict__ cta_panel,
     load(ca, wa, sb);
     if (hd < sb) cur = anb_pc_row(anb_ls_h(col + 32ll * hd + lane), anb_w1(w + 32ll * hd + lane), w);
   }
+  wait();
+  if (threadIdx.x == 0 && cw4 > 0) anb_bulk_issue(xs, x + c0, 4u * (unsigned)cw4, &anb_pc_mbar);
+  for (int q = cw4 + threadIdx.x; q < cw; q += blockDim.x) xs[q] = x[c0 + q];
   __syncthreads();                                   // mbarrier and tail rates published
   if (cw4 > 0) anb_bulk_wait(&anb_pc_mbar, err);
   for (int j = sb; j < se; j += 2 * U) {
