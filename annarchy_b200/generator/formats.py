@@ -292,11 +292,32 @@ def select_format(proj, compiled) -> str:
                 proj._sell_sigma = s["sell_sigma"]
             if "bsr_tile" in s:
                 proj._bsr_tile_size = s["bsr_tile"]
+            if s["format"] == "csr" and panels_pay(m):
+                return "pcsr"
             return s["format"]
     mean = m.nnz / max(1, (np.diff(m.indptr) > 0).sum())
     if mean <= 128:
         return "ellr" if proj.plastic else "sell"
     return "csr"
+
+
+def panels_pay(m) -> bool:
+    """Panels instead of CSR in a simulation. The selector's timings start with
+    a cold L2, which hides that CSR gathers the rates through L1 and L2; step
+    after step the matrix comes from L2 and the gathers are the bound, and a
+    panel's rates lie in shared memory. Measured per step of the launch plan
+    (CSR, panels): 3.8M synapses of 38,000 neurons 21.1, 11.9 us; 1.0M of
+    24,000 12.2, 8.8; 1.3M of 60,000 14.5, 9.8; 1.7M of 120,000 (8 panels) 21.4,
+    14.2; 23M of 120,000 110, 38. Below about 0.6M the launches are the time
+    (0.46M 10.6, 10.7), and a CSR projection can share the launch of a panelled
+    one (as the input projection did in the panelled runs). Above 32M synapses
+    (laying out the panels takes 0.1 s per million) the selector decides; rows
+    long enough for a CTA of their own stay with CSR's two kernels."""
+    if not (1 << 20) <= m.nnz <= (1 << 25):
+        return False
+    lengths = np.diff(m.indptr)
+    panels = -(-m.shape[1] // 16384)
+    return m.nnz >= 1.5 * panels * max(1, (lengths > 0).sum()) and csr_bins(m.indptr)[1].size == 0
 
 
 def create_format_arrays(compiled, proj, fmt, post_rank, row_ptr, cols, w, lay):
