@@ -9,7 +9,11 @@ Configuration (``Network.config``):
   precision    "double" (default): reference operation order, bit-identical
                results; "float": fast single-precision kernels.
   weight_dtype "float32" or "bfloat16" storage of static weights (float mode).
-  engine       "auto" | "grid" | "local" (see annarchy_b200.generator.codegen).
+  engine       "auto" | "grid" | "local" (see annarchy_b200.generator.codegen);
+               "auto" keeps small networks on chip for a whole run.
+  cluster_size CTAs of the cluster that such a spiking network runs on
+               (default: chosen by size).
+  resident_ctas  the same for a rate-coded network.
   graph_steps  steps captured per CUDA graph in the grid engine.
   pdl          True (default) | False: launch the grid engine's step kernels
                with programmatic dependent launch (each may be scheduled

@@ -1272,7 +1272,7 @@ def main():
             "frac": achieved / peak, "traffic": NCU_TRAFFIC.get((kname, "double")),
             "peak_source": peak_kind, "algorithmic_bytes_per_launch": abytes, "launch_ms": k_ms,
             "note": "10,000 dependent time steps of 4000 neurons in one launch: bound by the "
-                    "per-step cluster barrier and on-chip latency, not by HBM"}
+                    "per-step spike exchange and on-chip latency, not by HBM"}
 
     def e2e_run(net, P, mon, dtype):
         """Per step through the public API: initial state from pinned host
