@@ -601,7 +601,7 @@ class CodeGenerator:
         if ((threadIdx.x & 31) == 0 && {widx} < {lim}) {spk_dst}[{widx} >> 5] = anb_m;{recs}
       }}"""
         nl = "\n        "
-        keep, events = self._fused_post_events(pop, K) if grid_path and spiking else ("", "")
+        keep, events = self._fused_post_events(pop) if grid_path and spiking else ("", "")
         if keep:
             ballot = ballot.replace("__ballot_sync(0xffffffffu, anb_spiked);",
                                     "__ballot_sync(0xffffffffu, anb_spiked);" + keep.replace("anb_mw", "anb_m"), 1)
@@ -610,7 +610,7 @@ class CodeGenerator:
         const int anb_first = %s;"""
             shared = f"""
       __shared__ int anb_list[4 * ANB_DELIVER_LIST + 1];
-      __shared__ anb_u32 anb_sw[{BLOCK // 32 * K}];"""
+      __shared__ anb_u32 anb_sw[{BLOCK // 32}];"""
         else:
             events_pre, shared = "%.0s", ""
         if cluster is not None:
@@ -1914,8 +1914,13 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) anb_transmit() {{{''.join(
         kernel, in the CTA that updated the neuron that spiked: one launch per
         step less, and the spikes need not be found again. (Statements that
         read neurons' attributes keep their own kernel: other CTAs may still
-        be updating them.)"""
-        return self.fuse and self.own_post_events(proj)
+        be updating them.) Populations of 65,536 neurons and more keep it as well:
+        the spikes of a large population fall on few of its CTAs, and a kernel of
+        their own deals them out. 20,000 neurons 10.1 -> 7.5 us per step with
+        the fused form, 60,000 10.5 (own kernel) and 10.7, 200,000 13.1 and
+        15.7, 1M 24.6 and 29.6."""
+        return (self.fuse and self.own_post_events(proj)
+                and self.neurons_per_thread(proj.post_pop) == 1)
 
     def _post_args(self, proj) -> list:
         return [p["name"] for p in proj.desc["parameters"] + proj.desc["variables"]
@@ -1947,26 +1952,23 @@ __device__ __noinline__ anb_tr{k} proj{k}_post_syn(anb_tr{k} anb_s, const long l
         args = "".join(", " + n for n in self._post_args(proj))
         return f"proj{proj.id}_post_syn({record}, {t}, dt, anb_plastic{args})"
 
-    def _fused_post_events(self, pop, K: int) -> tuple[str, str]:
+    def _fused_post_events(self, pop) -> tuple[str, str]:
         """(shared memory and its use after each ballot, post events after the
         passes of one grid-stride iteration) of a population's update kernel."""
         projs = [p for p in self.net.projections if p.post_pop is pop and self.post_fused(p)]
         if not projs:
             return "", ""
-        words = BLOCK // 32 * K
+        words = BLOCK // 32
         keep = f"""
-        if ((threadIdx.x & 31) == 0) anb_sw[(anb_base - anb_first) / 32 + (threadIdx.x >> 5)] = anb_mw;
+        if ((threadIdx.x & 31) == 0) anb_sw[threadIdx.x >> 5] = anb_mw;
         anb_any |= anb_mw;"""
         parts = []
         for proj in projs:
             p = lambda n, k=proj.id: self.ptr(f"proj{k}__{n}")
             k = proj.id
             known = "\n          ".join(f"const {ct} {n} = anb_c{k}_{n};" for ct, n, _ in self._constants(proj))
-            find = f"""const int anb_ns = anb_list_spikes(anb_list, anb_sw, 0, anb_first / 32, {words}, 0, t, 0, {words},
-                                             {p('row_ptr')}, {p('row_of')});"""
-            if K == 1:
-                # (a population with one neuron per thread is one pass of the grid)
-                find = f"""const int anb_ns = anb_list_ranges(anb_list, (threadIdx.x & 31) < {words} ? anb_sw[threadIdx.x & 31] : 0u,
+            # (a population with one neuron per thread is one pass of the grid)
+            find = f"""const int anb_ns = anb_list_ranges(anb_list, (threadIdx.x & 31) < {words} ? anb_sw[threadIdx.x & 31] : 0u,
                                              anb_i0, anb_rb{k}, anb_re{k});"""
             parts.append(f"""
         {{  // {proj.name}
@@ -1999,15 +2001,13 @@ __device__ __noinline__ anb_tr{k} proj{k}_post_syn(anb_tr{k} anb_s, const long l
         if pop.id in getattr(self.c, "owned", {}):
             first, n = self.c.owned[pop.id]
         projs = [p for p in self.net.projections if p.post_pop is pop and self.post_fused(p)]
-        rows = projs and self.neurons_per_thread(pop) == 1
-        if rows:
+        if projs:
             out.append(f"const int anb_i0 = {first} + blockIdx.x * blockDim.x + threadIdx.x;")
         for proj in projs:
             k = proj.id
             p = lambda n, k=k: self.ptr(f"proj{k}__{n}")
             out += [f"const {ct} anb_c{k}_{nm} = {src}[0];" for ct, nm, src in self._constants(proj)]
-            if rows:
-                out.append(f"""int anb_rb{k} = 0, anb_re{k} = 0;
+            out.append(f"""int anb_rb{k} = 0, anb_re{k} = 0;
     {{
       const int anb_r = anb_i0 < {n} ? {p('row_of')}[anb_i0] : -1;
       if (anb_r >= 0) {{ anb_rb{k} = {p('row_ptr')}[anb_r]; anb_re{k} = {p('row_ptr')}[anb_r + 1]; }}
