@@ -85,15 +85,20 @@ class Masks:
     def slots(self):
         """Projections grouped into mask tables: one joins the table before it
         when both populations are the same and their pre-synaptic words are
-        disjoint. Tables keep the projections' order."""
+        disjoint. Tables keep the projections' order. Without delays the
+        projections of a table are added round by round, so that two of one
+        target would mix their additions: each then has its own table. (With
+        delays the events are counted and added projection by projection.)"""
         out = []
+        delayed = any(p.max_delay > 1 for p in self.net.projections)
         for p in self.net.projections:
             lay = self.c.layout[p.id]
             w0, w1 = lay["w0"], lay["w1"]
             if out:
                 s = out[-1]
                 if s["pre"] is p.pre_pop and s["post"] is p.post_pop and all(
-                        w1 <= a or b <= w0 for _, a, b in s["projs"]):
+                        (w1 <= a or b <= w0) and (delayed or q.target != p.target)
+                        for q, a, b in s["projs"]):
                     s["projs"].append((p, w0, w1))
                     s["w0"], s["w1"] = min(s["w0"], w0), max(s["w1"], w1)
                     continue
