@@ -492,7 +492,7 @@ class BatchGenerator(CodeGenerator):
             scratch += f"\n    if (threadIdx.x == 0) anb_lcnt[0] = anb_lcnt[1] = {self.b.list_cap} + 1;"
         src = f"""
 extern "C" __global__ void __launch_bounds__({BATCH_BLOCK}, 1)
-anb_batch_run(long long t0, int nsteps) {{
+anb_batch_run(long long anb_t0, int anb_steps) {{
     extern __shared__ __align__(16) unsigned char anb_smem[];
     const {dt_t} dt = ({dt_t})(*{self.ptr('dt')});
     const int anb_lane = threadIdx.x & 31;
@@ -509,8 +509,8 @@ anb_batch_run(long long t0, int nsteps) {{
       {load}
     }}
     __syncthreads();
-    for (int anb_s = 0; anb_s < nsteps; ++anb_s) {{
-      const long long t = t0 + anb_s;
+    for (int anb_s = 0; anb_s < anb_steps; ++anb_s) {{
+      const long long t = anb_t0 + anb_s;
       {deliver}
       __syncthreads();
       for (int anb_si = anb_sb; anb_si < anb_se; ++anb_si) {{
@@ -523,7 +523,7 @@ anb_batch_run(long long t0, int nsteps) {{
       {header}
       {store}
     }}
-    if (blockIdx.x == 0 && threadIdx.x == 0) *{self.ptr('t')} = t0 + nsteps;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *{self.ptr('t')} = anb_t0 + anb_steps;
 }}
 """
         return Module(self.assemble([src]), self.options(), "batch",

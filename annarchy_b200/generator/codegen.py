@@ -2132,7 +2132,7 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) mon{m}_record{'_targets' i
 
     def persistent_module(self) -> Module:
         """The grid engine's step as one cooperative persistent kernel
-        anb_grid_run(t0, nsteps): every kernel of the step plan becomes a
+        anb_grid_run(anb_t0, anb_steps): every kernel of the step plan becomes a
         device function; per step the functions run in plan order, the
         concurrent group of atomic transmissions as one phase, with a
         grid-wide barrier after every phase (bounded: a CTA that waits about
@@ -2182,22 +2182,22 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) mon{m}_record{'_targets' i
         bodies += [self.fused_stdp_functions(p) for p in fused]
         # the post events of the last step (the next launch starts unfused):
         # proj<k>_post_event_body, converted with the plan's other kernels
-        tail = "".join(f"\n      proj{p.id}_post_event_body(t0 + nsteps - 1);" for p in fused)
+        tail = "".join(f"\n      proj{p.id}_post_event_body(anb_t0 + anb_steps - 1);" for p in fused)
         # one CTA of PERSISTENT_BLOCK threads per SM: few CTAs arrive at each
         # grid barrier (the arrivals serialise on one counter)
         src = f"""
-extern "C" __global__ void __launch_bounds__({PERSISTENT_BLOCK}, 1) anb_grid_run(long long t0, int nsteps) {{
+extern "C" __global__ void __launch_bounds__({PERSISTENT_BLOCK}, 1) anb_grid_run(long long anb_t0, int anb_steps) {{
     int anb_s = 0;
-    for (; anb_s < nsteps; ++anb_s) {{
-      const long long t = t0 + anb_s;
+    for (; anb_s < anb_steps; ++anb_s) {{
+      const long long t = anb_t0 + anb_s;
       // this step's spike lists start empty (their parity was last read by
       // the transmissions of step t - 1 and the post events of step t - 2)
       if (blockIdx.x == 0 && threadIdx.x == 0) {{{resets}
       }}{''.join(steps)}
     }}
-    if (anb_s == nsteps && nsteps > 0) {{{tail}
+    if (anb_s == anb_steps && anb_steps > 0) {{{tail}
     }}
-    if (blockIdx.x == 0 && threadIdx.x == 0 && anb_s == nsteps) *{t_ptr} = t0 + nsteps;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && anb_s == anb_steps) *{t_ptr} = anb_t0 + anb_steps;
 }}
 """
         return Module(self.assemble(bodies + [src]), self.options(), "grid",
@@ -2495,7 +2495,7 @@ extern "C" __global__ void anb_tick() {
         dt_t = "double" if self.exact else "float"
         nl = "\n    "
         src = f"""
-extern "C" __global__ void __launch_bounds__({block}, 1) anb_local_run(long long t0, int nsteps) {{
+extern "C" __global__ void __launch_bounds__({block}, 1) anb_local_run(long long anb_t0, int anb_steps) {{
     extern __shared__ __align__(16) unsigned char anb_smem[];
     const {dt_t} dt = ({dt_t})(*{self.ptr('dt')});
     const int anb_lane = threadIdx.x & 31;
@@ -2507,8 +2507,8 @@ extern "C" __global__ void __launch_bounds__({block}, 1) anb_local_run(long long
     {mon_pre}
     {nl.join(load)}
     __syncthreads();
-    for (int anb_s = 0; anb_s < nsteps; ++anb_s) {{
-      const long long t = t0 + anb_s;
+    for (int anb_s = 0; anb_s < anb_steps; ++anb_s) {{
+      const long long t = anb_t0 + anb_s;
       {''.join(prop)}
       __syncthreads();
       {''.join(updates)}
@@ -2517,7 +2517,7 @@ extern "C" __global__ void __launch_bounds__({block}, 1) anb_local_run(long long
     }}
     __syncthreads();
     {nl.join(store)}
-    if (threadIdx.x == 0) *{self.ptr('t')} = t0 + nsteps;
+    if (threadIdx.x == 0) *{self.ptr('t')} = anb_t0 + anb_steps;
 }}
 """
         return Module(self.assemble([src]), self.options(), "local",
@@ -2580,7 +2580,7 @@ extern "C" __global__ void __launch_bounds__({block}, 1) anb_local_run(long long
             # spikes of the step before the launch go to the replica of parity 1
             load.append(f"for (int q = threadIdx.x; q < {words}; q += blockDim.x) {{ {d['spk1']}[q] = {gspk}[q]; {d['spk0']}[q] = 0u; }}")
             store.append(f"for (int q = threadIdx.x; q < anb_words{k}; q += blockDim.x) "
-                         f"{gspk}[(anb_base{k} >> 5) + q] = (nsteps & 1 ? {d['spk0']} : {d['spk1']})[(anb_base{k} >> 5) + q];")
+                         f"{gspk}[(anb_base{k} >> 5) + q] = (anb_steps & 1 ? {d['spk0']} : {d['spk1']})[(anb_base{k} >> 5) + q];")
         prop = []
         fast_groups: dict[int, list] = {}
         exact_groups: dict[tuple, list] = {}
@@ -2727,7 +2727,7 @@ extern "C" __global__ void __launch_bounds__({block}, 1) anb_local_run(long long
         nl = "\n    "
         src = f"""
 extern "C" __global__ void __launch_bounds__({block}, 1)
-anb_cluster_run(long long t0, int nsteps) {{
+anb_cluster_run(long long anb_t0, int anb_steps) {{
     extern __shared__ __align__(16) unsigned char anb_smem[];
     const unsigned anb_rank = anb_cluster_rank();
     const {dt_t} dt = ({dt_t})(*{self.ptr('dt')});
@@ -2744,8 +2744,8 @@ anb_cluster_run(long long t0, int nsteps) {{
     {nl.join(load)}
     (void)anb_pool_off;
     anb_cluster_sync();
-    for (int anb_s = 0; anb_s < nsteps; ++anb_s) {{
-      const long long t = t0 + anb_s;
+    for (int anb_s = 0; anb_s < anb_steps; ++anb_s) {{
+      const long long t = anb_t0 + anb_s;
       const int anb_par = anb_s & 1;
       {''.join(prop)}
       __syncthreads();
@@ -2753,7 +2753,7 @@ anb_cluster_run(long long t0, int nsteps) {{
       anb_cluster_sync();
     }}
     {nl.join(store)}
-    if (anb_rank == 0 && threadIdx.x == 0) *{self.ptr('t')} = t0 + nsteps;
+    if (anb_rank == 0 && threadIdx.x == 0) *{self.ptr('t')} = anb_t0 + anb_steps;
 }}
 """
         return Module(self.assemble([src]), self.options(), "cluster",

@@ -275,7 +275,7 @@ class Masks:
             spk = gen.ptr(f"pop{k}__spk")
             ring = c.slots.get(k, 1)
             # the spikes before the run are read from the bitmaps in memory
-            last = f"{spk} + (size_t)anb_ring_slot(t0 - 1, {ring}) * {d['words']}"
+            last = f"{spk} + (size_t)anb_ring_slot(anb_t0 - 1, {ring}) * {d['words']}"
             load.append(f"#pragma unroll 1\n    for (int q = threadIdx.x; q < {32 * d['per']}; q += {block}) {{ "
                         f"anb_rep{k}1[q] = q < {d['words']} ? ({last})[q] : 0u; anb_rep{k}0[q] = 0u; }}")
             if ring > 1:
@@ -284,11 +284,11 @@ class Masks:
             if lists and lay["S"]:
                 # (the grid engine's spike lists are emptied when the time is set)
                 spn = gen.ptr(f"pop{k}__spn")
-                regs.append(f"const bool anb_had{k} = {spn}[(t0 - 1) & 1] != 0;")
+                regs.append(f"const bool anb_had{k} = {spn}[(anb_t0 - 1) & 1] != 0;")
                 store.append(f"if (anb_rank == 0 && threadIdx.x < 2) {spn}[threadIdx.x] = 1;")
             if ring == 1:
                 store.append(f"if (anb_tid < anb_cnt{k} && anb_lane == 0) {spk}[(anb_base{k} + anb_tid) >> 5] = "
-                             f"(nsteps & 1 ? anb_rep{k}0 : anb_rep{k}1)[(anb_base{k} + anb_tid) >> 5];")
+                             f"(anb_steps & 1 ? anb_rep{k}0 : anb_rep{k}1)[(anb_base{k} + anb_tid) >> 5];")
             smem = {}
             names = [(n, R) for n in c._local_vars(pop)] + [("refractory_remaining", "int")]
             if pop._has_refractory:
@@ -447,7 +447,7 @@ class Masks:
         globals_ = [gen._globals_preamble(p, lambda n, kk=p.id: gen.ptr(f"pop{kk}__{n}")) for p in net.populations]
         mon_pre = "\n    ".join(
             f"const int anb_mon_on{m.id} = {gen.ptr(f'mon{m.id}__on')}[0];\n    "
-            f"const long long anb_sl{m.id} = t0 - {gen.ptr(f'mon{m.id}__t0')}[0];\n    "
+            f"const long long anb_sl{m.id} = anb_t0 - {gen.ptr(f'mon{m.id}__t0')}[0];\n    "
             f"const int anb_slot0{m.id} = anb_sl{m.id} < -(1 << 30) || anb_sl{m.id} > (1 << 30) ? -(1 << 30) : (int)anb_sl{m.id};"
             for m in net.monitors)
         dt_t = "double" if c.exact else "float"
@@ -456,15 +456,15 @@ class Masks:
             warps = f"max({warps}, anb_cnt{p.id})"
         # with delays the steps before the run that still matter come first
         S = lay["S"]
-        start = f"nsteps > 0 ? {2 - S} : 0" if S else "0"
+        start = f"anb_steps > 0 ? {2 - S} : 0" if S else "0"
         # (positions in the rings are counted: a 64-bit remainder is 100 cycles)
         cursor = f"""
         anb_cur = anb_cur + 1 == {S} ? 0 : anb_cur + 1;""" if S else ""
-        rings = f"int anb_cur = anb_ring_slot(t0 + ({start}) - 1, {S});" if S else ""
+        rings = f"int anb_cur = anb_ring_slot(anb_t0 + ({start}) - 1, {S});" if S else ""
         for pop in net.populations:
             ring = c.slots.get(pop.id, 1)
             if ring > 1:
-                rings += f"\n      int anb_at{pop.id} = anb_ring_slot(t0 + ({start}) - 1, {ring});"
+                rings += f"\n      int anb_at{pop.id} = anb_ring_slot(anb_t0 + ({start}) - 1, {ring});"
                 cursor += f"""
         anb_at{pop.id} = anb_at{pop.id} + 1 == {ring} ? 0 : anb_at{pop.id} + 1;"""
         skip = """
@@ -473,7 +473,7 @@ class Masks:
         nl = "\n    "
         err = gen.ptr("err")
         src = f"""
-extern "C" __global__ void __launch_bounds__({block}, 1) anb_cluster_run(long long t0, int nsteps) {{
+extern "C" __global__ void __launch_bounds__({block}, 1) anb_cluster_run(long long anb_t0, int anb_steps) {{
     extern __shared__ __align__(16) unsigned char anb_smem[];
     const unsigned anb_rank = anb_cluster_rank();
     const {dt_t} dt = ({dt_t})(*{gen.ptr('dt')});
@@ -502,8 +502,8 @@ extern "C" __global__ void __launch_bounds__({block}, 1) anb_cluster_run(long lo
     if (anb_warp < anb_warps) {{
       {rings}
 #pragma unroll 1
-      for (int anb_s = {start}; anb_s < nsteps; ++anb_s) {{
-        const long long t = t0 + anb_s;{cursor}
+      for (int anb_s = {start}; anb_s < anb_steps; ++anb_s) {{
+        const long long t = anb_t0 + anb_s;{cursor}
         if (anb_s > 0) {{
           // the words of step s - 1; the barrier's next phase takes those of s + 1
           const unsigned b = anb_bar + 8u * ((anb_s - 1) & 1);
@@ -515,12 +515,12 @@ extern "C" __global__ void __launch_bounds__({block}, 1) anb_cluster_run(long lo
         if (anb_lane == 0) anb_mbar_arrive(anb_bar + 8u * (anb_s & 1));
       }}
       // the last step's words have arrived everywhere before any CTA leaves
-      if (nsteps > 0) anb_mbar_wait(anb_bar + 8u * ((nsteps - 1) & 1), ((nsteps - 1) >> 1) & 1, {err});
+      if (anb_steps > 0) anb_mbar_wait(anb_bar + 8u * ((anb_steps - 1) & 1), ((anb_steps - 1) >> 1) & 1, {err});
       {nl.join(store)}
     }}
     __syncwarp();
     anb_cluster_sync();
-    if (anb_rank == 0 && threadIdx.x == 0) *{gen.ptr('t')} = t0 + nsteps;
+    if (anb_rank == 0 && threadIdx.x == 0) *{gen.ptr('t')} = anb_t0 + anb_steps;
 }}
 """
         return Module(gen.assemble([src]), gen.options(), "cluster",

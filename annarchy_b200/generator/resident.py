@@ -336,7 +336,7 @@ class Resident:
         nl = "\n    "
         name = "anb_rate_run"
         src = f"""
-extern "C" __global__ void __launch_bounds__({BLOCK}, 1) {name}(long long t0, int nsteps) {{
+extern "C" __global__ void __launch_bounds__({BLOCK}, 1) {name}(long long anb_t0, int anb_steps) {{
     extern __shared__ __align__(16) unsigned char anb_smem[];
     {guard}const int anb_rank = {rank};
     const {dt_t} dt = ({dt_t})(*{gen.ptr('dt')});
@@ -349,14 +349,14 @@ extern "C" __global__ void __launch_bounds__({BLOCK}, 1) {name}(long long t0, in
     {nl.join(load)}{''.join(fill)}
     {first}
 #pragma unroll 1
-    for (int anb_s = 0; anb_s < nsteps; ++anb_s) {{
-      const long long t = t0 + anb_s;
+    for (int anb_s = 0; anb_s < anb_steps; ++anb_s) {{
+      const long long t = anb_t0 + anb_s;
       {''.join(recs)}{''.join(steps)}
       {meet}
     }}
     __syncthreads();
     {nl.join(store)}
-    if (anb_rank == 0 && threadIdx.x == 0) *{gen.ptr('t')} = t0 + nsteps;
+    if (anb_rank == 0 && threadIdx.x == 0) *{gen.ptr('t')} = anb_t0 + anb_steps;
 }}
 """
         smem_bytes = lay["smem"] if cluster else max(lay["smem"], SMEM_ALONE)
