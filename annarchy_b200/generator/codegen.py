@@ -359,6 +359,21 @@ class CodeGenerator:
                 out.append(self.typed(f"const double {pl['name']} = {self.fill(pl['value'])};"))
         return "\n    ".join(out)
 
+    def _scoped_globals(self, pop) -> tuple[str, str]:
+        """The same for a kernel of many steps and several populations, whose
+        values may share names: loads under names of their own before the step
+        loop, and the names the equations use, for the population's block."""
+        loads = self._globals_preamble(pop, lambda n: self.ptr(f"pop{pop.id}__{n}")).split("\n    ")
+        own = {}
+        for i, line in enumerate(x for x in loads if x):
+            kind, name, value = re.fullmatch(r"((?:const )?\w+) (\w+) = (.*);", line).groups()
+            for n, (_, g) in own.items():
+                value = re.sub(rf"\b{n}\b", g, value)
+            own[name] = (kind, f"anb_g{pop.id}_{name}")
+            loads[i] = f"{kind} {own[name][1]} = {value};"
+        return ("\n    ".join(x for x in loads if x),
+                " ".join(f"{kind} {n} = {g};" for n, (kind, g) in own.items()))
+
     _DRAW_FN = {"Uniform": "anb_draw_uniform", "Normal": "anb_draw_normal",
                 "LogNormal": "anb_draw_lognormal", "Exponential": "anb_draw_exponential",
                 "DiscreteUniform": "anb_draw_discrete_uniform"}
@@ -2685,7 +2700,8 @@ extern "C" __global__ void __launch_bounds__({block}, 1) anb_local_run(long long
         updates, globals_, bcast, recs = [], [], [], []
         for pop in net.populations:
             k = pop.id
-            globals_.append(self._globals_preamble(pop, lambda n, kk=k: self.ptr(f"pop{kk}__{n}")))
+            before, inside = self._scoped_globals(pop)
+            globals_.append(before)
             d = dict(smem_ptrs[k])
             # right after its ballot, a warp stores its bitmap word into every
             # CTA's replica (lane r -> CTA r) and one lane records it
@@ -2713,8 +2729,8 @@ extern "C" __global__ void __launch_bounds__({block}, 1) anb_local_run(long long
           else if (anb_lane < {C}) anb_cluster_st_u32(anb_cluster_map(anb_smem_addr(anb_dstw), (unsigned)anb_lane), anb_m);{rec}
         }}
       }}"""
-            updates.append(self.neuron_update(pop, local_engine=True, smem=d, cluster={},
-                                              ballot_hook=hook))
+            updates.append(f"{{ {inside}" + self.neuron_update(pop, local_engine=True, smem=d, cluster={},
+                                                              ballot_hook=hook) + "}")
         mon_pre = "\n    ".join(
             f"const int anb_mon_on{mon.id} = {self.ptr(f'mon{mon.id}__on')}[0];\n    "
             f"const long long anb_mon_t0{mon.id} = {self.ptr(f'mon{mon.id}__t0')}[0];"

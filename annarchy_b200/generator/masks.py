@@ -444,7 +444,7 @@ class Masks:
             __syncwarp();
           }}{drain}
         }}"""
-        globals_ = [gen._globals_preamble(p, lambda n, kk=p.id: gen.ptr(f"pop{kk}__{n}")) for p in net.populations]
+        globals_ = [gen._scoped_globals(p)[0] for p in net.populations]
         mon_pre = "\n    ".join(
             f"const int anb_mon_on{m.id} = {gen.ptr(f'mon{m.id}__on')}[0];\n    "
             f"const long long anb_sl{m.id} = anb_t0 - {gen.ptr(f'mon{m.id}__t0')}[0];\n    "
@@ -557,6 +557,7 @@ extern "C" __global__ void __launch_bounds__({block}, 1) anb_cluster_run(long lo
         }}
       }}"""
         code = gen.neuron_update(pop, local_engine=True, smem=smem, cluster={}, ballot_hook=hook)
+        code = f"{{ {gen._scoped_globals(pop)[1]}{code}}}"
         code = re.sub(r"(anb_rg\d+_\w+)\[anb_q\]", r"\1", code)
         code = code.replace("for (int anb_q0 = 0; anb_q0 < anb_cnt; anb_q0 += blockDim.x) {",
                             "{ const int anb_q0 = 0;")
