@@ -245,6 +245,8 @@ class Masks:
     def write_weights(self, proj) -> bool:
         """The weights set after compile(); False when they differ."""
         w = proj._csr.data
+        if not w.size:
+            return True
         if not np.all(w == w[0]):
             return False
         self.c.native.write(f"proj{proj.id}__mw", self.c._w(np.array([w[0]])))
