@@ -1082,6 +1082,9 @@ class CompiledNetwork:
     def write_population_attribute(self, pop, name, arr):
         dt = np.int32 if pop._host[name].dtype == np.int32 else self.real
         self.native.write(f"pop{pop.id}__{name}", np.asarray(arr, dtype=dt).reshape(-1))
+        if name in compensated_vars(pop, self.exact, self.net._config):
+            # (the carried rounding error is that of the former value)
+            self.native.fill(f"pop{pop.id}__kc_{name}", self.real(0))
 
     def write_refractory(self, pop):
         self.native.write(f"pop{pop.id}__refractory", pop.refractory_steps.astype(np.int32))
