@@ -239,11 +239,14 @@ class CompiledNetwork:
         return False
 
     def _leave_masks(self):
-        """From the cluster form of a delayed network to the grid engine's
-        plan, which reads the same bitmaps and states: its projections now
-        carry different weights."""
+        """From the mask kernel to the form for projections with several
+        weights, which reads the same bitmaps and states: with delays the grid
+        engine's plan, without them the cluster kernel with synapse lists."""
         nat = self.native
         self.masks = None
+        if self.engine == "cluster":
+            self._build_cluster_lists()
+            return
         self._build_plan()
         t = nat.get_time()
         for pop in self.net.populations:
@@ -265,11 +268,16 @@ class CompiledNetwork:
         cluster (up to 16 CTAs) whose shared memory holds the state and the
         synapses; otherwise 8 CTAs with the synapses read from global memory.
         A cluster the device cannot schedule falls back the same way."""
-        from ..runtime.lib import BackendError
         masks = Masks(self)
         if masks.possible() and self._load_masks(masks):
+            self.masks = masks
             self.engine = "cluster"
             return
+        self._build_cluster_lists()
+
+    def _build_cluster_lists(self):
+        """The cluster kernel whose CTAs hold lists of their synapses."""
+        from ..runtime.lib import BackendError
         want = self.net._config.get("cluster_size")
         total = max(p.size for p in self.net.populations)
         cands = [int(want)] if want else [c for c in (1, 2, 4, 8, 16) if (total + c - 1) // c <= 1024]
@@ -298,6 +306,27 @@ class CompiledNetwork:
             self.engine = "cluster"
             return
         raise RuntimeError(f"no cluster configuration fits this network ({last_err})")
+
+    def _write_cluster_weights(self, proj):
+        """The weights set after compile() into the cluster kernel's synapse
+        lists (as indices into the table of its distinct weights where it has
+        one; a longer table needs another layout)."""
+        k, lay = proj.id, self.cluster_layout
+        pl = self.layout[k]
+        arrs = self._incoming_slices(proj, lay["C"], lay["pops"][proj.post_pop.id]["chunk"], pl["w0"] * 32,
+                                     (pl["w1"] - pl["w0"]) * 32)
+        w = arrs["cl_w"]
+        put = (lambda a: a) if self.exact else self._w
+        if lay["pool"]["palette"]:
+            n = lay["proj"][k]["pal"][1]
+            table = np.unique(w)
+            if table.size > n:
+                self._build_cluster_lists()
+                return
+            self.native.write(f"proj{k}__cl_wi", np.searchsorted(table, w).astype(np.uint8))
+            table = np.concatenate([table, np.zeros(n - table.size)])
+            self.native.write(f"proj{k}__cl_pal", put(table))
+        self.native.write(f"proj{k}__cl_w", put(w))
 
     def _setup_shard(self):
         from .shard import Exchange, owned_range
@@ -1220,6 +1249,8 @@ class CompiledNetwork:
         dtype, _ = self.native.arrays[f"proj{k}__{name}"]
         data = to_bf16(arr) if dtype == np.uint16 else np.asarray(arr, dtype=dtype)
         self.native.write(f"proj{k}__{name}", data)
+        if name == "w" and self.engine == "cluster" and self.masks is None:
+            self._write_cluster_weights(proj)
         if name == "w" and f"proj{k}__w_pre" in self.native.arrays:
             order = self.native.read(f"proj{k}__inv_idx")
             dtype, _ = self.native.arrays[f"proj{k}__w_pre"]
