@@ -180,6 +180,7 @@ struct anb_net {
   // pinned staging of kStage bytes for device-to-host copies, then as many for
   // decoded spikes
   unsigned char* stage = nullptr;
+  std::recursive_mutex stage_mutex; // held while the stage or the decoder's scratch is in use
   // stop conditions of populations (anb_run_until): the kernel of population
   // `pop` writes the device step into stop_flags[pop] when a neuron satisfies
   // the condition ("any") or when one fails it ("all")
@@ -515,12 +516,17 @@ void give_stage(anb_net* net) {
 // to every page first: the driver is slow on pages that do not exist yet (256 MB
 // into a new array 54 ms, 41 this way and 43 through the stage).
 int read_staged(anb_net* net, const void* src, void* dst, size_t bytes) {
-  void* to = bytes <= kStage ? (void*)net->stage : dst;
-  if (to == dst)
+  if (bytes > kStage) {
     for (size_t off = 0; off < bytes; off += 4096) static_cast<volatile unsigned char*>(dst)[off] = 0;
-  ANB_CUDA(cudaMemcpyAsync(to, src, bytes, cudaMemcpyDeviceToHost, net->stream));
+    ANB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, net->stream));
+    ANB_CUDA(cudaStreamSynchronize(net->stream));
+    return ANB_OK;
+  }
+  // (several threads may read one network's arrays)
+  std::lock_guard<std::recursive_mutex> lock(net->stage_mutex);
+  ANB_CUDA(cudaMemcpyAsync(net->stage, src, bytes, cudaMemcpyDeviceToHost, net->stream));
   ANB_CUDA(cudaStreamSynchronize(net->stream));
-  if (to != dst) std::memcpy(dst, to, bytes);
+  std::memcpy(dst, net->stage, bytes);
   return ANB_OK;
 }
 
@@ -1110,6 +1116,7 @@ int anb_monitor_decode_slots(anb_net* net, const char* array, int64_t steps, int
       return fail(ANB_ERR_ARG, "slots must be ascending ranges of the ring's words");
   int rc = ensure_device(net);
   if (rc) return rc;
+  std::lock_guard<std::recursive_mutex> lock(net->stage_mutex);
   net->dec_last = net->dec_ready = 0;
   for (int64_t i = 0; i <= n_slots; ++i) offsets[i] = 0;
   if (steps == 0) return ANB_OK;
@@ -1182,6 +1189,7 @@ int anb_monitor_fetch(anb_net* net, int64_t first_step, int64_t* out_steps, int6
                       int64_t count) {
   if (!net || count < 0 || (count > 0 && (!out_steps || !out_ranks)))
     return fail(ANB_ERR_ARG, "bad argument");
+  std::lock_guard<std::recursive_mutex> lock(net->stage_mutex);
   if (count > net->dec_last) return fail(ANB_ERR_ARG, "more spikes requested than were decoded");
   int rc = ensure_device(net);
   if (rc) return rc;
@@ -1209,6 +1217,7 @@ int anb_monitor_decode(anb_net* net, const char* array, int64_t steps, int64_t w
   const int64_t first[2] = {0, words_per_step};
   int64_t off[2] = {0, 0};
   *count = 0;
+  std::lock_guard<std::recursive_mutex> lock(net->stage_mutex);
   int rc = anb_monitor_decode_slots(net, array, steps, words_per_step, n, 1, first, off);
   if (rc) return rc;
   *count = off[1];
