@@ -300,8 +300,8 @@ class Masks:
                 reg = f"anb_rg{k}_{n}"
                 smem[n] = reg
                 regs.append(f"{ct} {reg} = ({ct})0;")
-                if n.startswith("kc_"):
-                    continue
+                if n.startswith("kc_") and not lay["S"]:
+                    continue        # without delays a run starts without carried errors
                 g = gen.ptr(f"pop{k}__{n}")
                 load.append(f"if (anb_tid < anb_cnt{k}) {reg} = {g}[anb_base{k} + anb_tid];")
                 if n != "refractory":
