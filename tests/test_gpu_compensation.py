@@ -1,6 +1,7 @@
 """Compensated variables in single precision: a value that is set is the
 value, without the rounding error carried for the former one; the errors last
 from run to run."""
+import numpy as np
 import pytest
 
 import annarchy_b200 as ann
