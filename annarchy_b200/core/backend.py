@@ -460,7 +460,7 @@ class CompiledNetwork:
             words = (pop.size + 31) // 32
             d = {}
             for name in self._local_vars(pop):
-                d[name] = (off, rct)
+                d[name] = (off, "int" if pop._ctype.get(name) in ("int", "bool") else rct)
                 off += a16(chunk * rb)
             d["refractory_remaining"] = (off, "int")
             off += a16(chunk * 4)

@@ -292,7 +292,8 @@ class Masks:
                 store.append(f"if (anb_tid < anb_cnt{k} && anb_lane == 0) {spk}[(anb_base{k} + anb_tid) >> 5] = "
                              f"(anb_steps & 1 ? anb_rep{k}0 : anb_rep{k}1)[(anb_base{k} + anb_tid) >> 5];")
             smem = {}
-            names = [(n, R) for n in c._local_vars(pop)] + [("refractory_remaining", "int")]
+            names = [(n, "int" if pop._ctype.get(n) in ("int", "bool") else R) for n in c._local_vars(pop)]
+            names.append(("refractory_remaining", "int"))
             if pop._has_refractory:
                 names.append(("refractory", "int"))
             names += [("kc_" + n, R) for n in compensated_vars(pop, c.exact, net._config)]
