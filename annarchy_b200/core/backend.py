@@ -150,13 +150,7 @@ class CompiledNetwork:
         if self.engine == "local":
             self._build_cluster()
             return
-        if resident:
-            res, lay = resident
-            res.create_arrays(lay)
-            self.module = res.module(lay)
-            nat.load_module(self.module.source, self.module.options)
-            self.write_constants()
-            nat.set_local_kernel(*self.module.local)
+        if resident and self._load_resident(*resident):
             return
         self._build_plan()
 
@@ -228,14 +222,38 @@ class CompiledNetwork:
         for lay in masks.choose():
             masks.create_arrays(lay)
             mod = masks.module(lay)
+            self.native.load_module(mod.source, mod.options)
+            self.write_constants()
             try:
-                self.native.load_module(mod.source, mod.options)
-                self.write_constants()
                 self.native.set_local_kernel(*mod.local)
             except BackendError:
-                continue                       # a cluster the device cannot schedule
+                masks.free_arrays()            # a cluster the device cannot schedule
+                continue
             self.module = mod
             return True
+        return False
+
+    def _load_resident(self, res, lay) -> bool:
+        from ..runtime.lib import BackendError
+        nat = self.native
+        before = set(nat.arrays)
+        res.create_arrays(lay)
+        self.module = res.module(lay)
+        nat.load_module(self.module.source, self.module.options)
+        self.write_constants()
+        try:
+            nat.set_local_kernel(*self.module.local)
+            if lay["cluster"] or getattr(nat, "local_grid", lay["ctas"]) >= lay["ctas"]:
+                return True
+        except BackendError:
+            pass
+        # CTAs that the device cannot schedule together: the launch plan, with
+        # the storage formats it chooses
+        for name in set(nat.arrays) - before:
+            nat.free(name)
+        self.engine = "grid"
+        for proj in self.net.projections:
+            self._create_projection(proj)
         return False
 
     def _leave_masks(self):
@@ -243,11 +261,13 @@ class CompiledNetwork:
         weights, which reads the same bitmaps and states: with delays the grid
         engine's plan, without them the cluster kernel with synapse lists."""
         nat = self.native
-        self.masks = None
+        masks, self.masks = self.masks, None
         if self.engine == "cluster":
             self._build_cluster_lists()
+            masks.free_arrays()
             return
         self._build_plan()
+        masks.free_arrays()
         t = nat.get_time()
         for pop in self.net.populations:
             name = f"pop{pop.id}__spn"

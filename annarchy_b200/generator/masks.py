@@ -193,6 +193,10 @@ class Masks:
             self._delay_arrays(i, s, lay, nat.create)
         self.lay = lay
 
+    def free_arrays(self):
+        for name in [n for n in self.c.native.arrays if n.startswith("net__") or n.endswith("__mw")]:
+            self.c.native.free(name)
+
     def _delay_arrays(self, i, slot, lay, put):
         if slot["packed"]:
             positions, delays = slot.pop("arrays", None) or self.packed(slot, lay)
