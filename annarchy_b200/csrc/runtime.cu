@@ -177,9 +177,9 @@ struct anb_net {
   int64_t dec_ready = 0;            // of these, in the stage's second half
   long long* dec_first = nullptr;   // first word of every slot
   int64_t dec_first_cap = 0;
-  // pinned staging of kStage bytes for device-to-host copies, then as many for
-  // decoded spikes
+  // pinned staging for device-to-host copies, two halves of kStage bytes
   unsigned char* stage = nullptr;
+  cudaEvent_t stage_ev[2] = {nullptr, nullptr};
   std::recursive_mutex stage_mutex; // held while the stage or the decoder's scratch is in use
   // stop conditions of populations (anb_run_until): the kernel of population
   // `pop` writes the device step into stop_flags[pop] when a neuron satisfies
@@ -479,6 +479,8 @@ std::mutex g_pin_mutex;
 std::vector<unsigned char*> g_pins;
 
 int take_stage(anb_net* net) {
+  for (auto& ev : net->stage_ev)
+    if (!ev) ANB_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   {
     std::lock_guard<std::mutex> lock(g_pin_mutex);
     if (!g_pins.empty()) {
@@ -508,15 +510,18 @@ void give_stage(anb_net* net) {
   cudaFreeHost(p);
 }
 
-// Device memory to the host after the stream's work. Up to kStage bytes go
-// through the pinned stage: a copy into pageable memory is staged by the driver
-// in the same way, with two more synchronisations (32 KB took 19 us and take 15,
-// 1 MB 87 and 77). Larger copies are the driver's (into memory in use 2 MB take
-// 143 us, and 160 through the stage in parts; 256 MB 13.7 and 22 ms), with a write
-// to every page first: the driver is slow on pages that do not exist yet (256 MB
-// into a new array 54 ms, 41 this way and 43 through the stage).
+// Device memory to the host after the stream's work. Up to kStaged bytes go
+// through the pinned stage, the copy of the next part while this one is moved to
+// dst: a copy into pageable memory is staged by the driver in the same way, with
+// two more synchronisations (32 KB took 19 us and take 15, 1 MB 87 and 77), and
+// leaves nothing in the caches for the conversion that follows most reads (5 MB of
+// packed weights and their widening: 1.5 and 2.1 ms). Larger copies are the driver's
+// (256 MB into memory in use 13.7 ms, 22 through the stage), with a write to every
+// page first: the driver is slow on pages that do not exist yet (256 MB into a
+// new array 54 ms, 41 this way and 43 through the stage).
+constexpr size_t kStaged = 16 << 20;
 int read_staged(anb_net* net, const void* src, void* dst, size_t bytes) {
-  if (bytes > kStage) {
+  if (bytes > kStaged) {
     for (size_t off = 0; off < bytes; off += 4096) static_cast<volatile unsigned char*>(dst)[off] = 0;
     ANB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, net->stream));
     ANB_CUDA(cudaStreamSynchronize(net->stream));
@@ -524,9 +529,21 @@ int read_staged(anb_net* net, const void* src, void* dst, size_t bytes) {
   }
   // (several threads may read one network's arrays)
   std::lock_guard<std::recursive_mutex> lock(net->stage_mutex);
-  ANB_CUDA(cudaMemcpyAsync(net->stage, src, bytes, cudaMemcpyDeviceToHost, net->stream));
-  ANB_CUDA(cudaStreamSynchronize(net->stream));
-  std::memcpy(dst, net->stage, bytes);
+  const size_t parts = (bytes + kStage - 1) / kStage;
+  if (parts > 1) net->dec_ready = 0;   // decoded pairs kept in the second half
+  auto issue = [&](size_t i) -> cudaError_t {
+    const size_t off = i * kStage, n = bytes - off < kStage ? bytes - off : kStage;
+    cudaError_t e = cudaMemcpyAsync(net->stage + (i & 1) * kStage, (const unsigned char*)src + off, n,
+                                    cudaMemcpyDeviceToHost, net->stream);
+    return e != cudaSuccess ? e : cudaEventRecord(net->stage_ev[i & 1], net->stream);
+  };
+  ANB_CUDA(issue(0));
+  for (size_t i = 0; i < parts; ++i) {
+    if (i + 1 < parts) ANB_CUDA(issue(i + 1));
+    ANB_CUDA(cudaEventSynchronize(net->stage_ev[i & 1]));
+    const size_t off = i * kStage, n = bytes - off < kStage ? bytes - off : kStage;
+    std::memcpy((unsigned char*)dst + off, net->stage + (i & 1) * kStage, n);
+  }
   return ANB_OK;
 }
 
@@ -631,6 +648,8 @@ int anb_destroy(anb_net* net) {
   if (net->dec_out) cudaFree(net->dec_out);
   if (net->dec_first) cudaFree(net->dec_first);
   give_stage(net);
+  for (auto ev : net->stage_ev)
+    if (ev) cudaEventDestroy(ev);
   if (net->module) g_drv.moduleUnload(net->module);
   for (auto& kv : net->arrays) cudaFree(kv.second.ptr);
   if (net->own_stream) cudaStreamDestroy(net->own_stream);
