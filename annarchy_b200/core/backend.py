@@ -70,6 +70,9 @@ class CompiledNetwork:
         self._exchange = None
         # projections delivered through per-neuron inboxes (double precision)
         self.inbox: set = set()
+        # population -> word ranges of its bitmap whose spikes are counted
+        # (first word, end, every how many words): see _create_inbox
+        self.activity: dict = {}
         # the cluster form with per-warp masks, when it runs the network
         self.masks = None
         # rate tiles of a RateBatch: population -> (first block column, neurons
@@ -139,6 +142,10 @@ class CompiledNetwork:
         self._batched_tiles()
         for proj in net.projections:
             self._create_projection(proj)
+        for k, ranges in self.activity.items():
+            # per range: the counts of the steps in the history and of the one under
+            # way, then (8-byte aligned) the sums over a history, by step parity
+            nat.create(f"pop{k}__nsp", np.zeros(len(ranges) * self.activity_stride(k), dtype=np.uint32))
         for mon in net.monitors:
             self._create_monitor(mon)
         for pop in net.populations:
@@ -687,7 +694,7 @@ class CompiledNetwork:
             row_of = np.full(proj.post_pop.size, -1, dtype=np.int32)
             row_of[post0:post0 + npost] = np.arange(npost, dtype=np.int32)
             nat.create(f"proj{k}__row_of", row_of)
-        self._create_inbox(proj, nnz)
+        self._create_inbox(proj, lay, post0 + np.arange(npost), lengths[row0:row0 + npost])
         if self.spike_lists:
             lay["grid"] = list_grid(pre_hi - pre_lo, lay["chunks"])
         elif self.exact or plastic:
@@ -714,21 +721,50 @@ class CompiledNetwork:
                 nat.fill(f"proj{k}___last_event", np.int64(-10000))
         self.layout[k] = lay
 
-    def _create_inbox(self, proj, nnz):
+    def activity_stride(self, k: int) -> int:
+        return (self.slots[k] + 2) // 2 * 2 + 2
+
+    def _create_inbox(self, proj, lay, posts, lengths):
         """Inbox of every post neuron (counter, entries), the copy of the
         bitmap words its row walk reads and, for plastic synapses, the value
-        each one transmitted (see anb_inbox_add)."""
+        each one transmitted (see anb_inbox_add). lay["dense"]: from how many
+        counted spikes on the rows are walked instead (see below); lay["act"]:
+        which of the population's counters counts them."""
         k = proj.id
         if k not in self.inbox:
             return
         nat = self.native
+        pre = proj.pre_pop.id
         n = proj.post_pop.size
         key = np.uint64 if proj._delay_steps is not None else np.uint32
         nat.create(f"proj{k}__ibn", np.zeros(n, dtype=np.uint32))
         nat.create_empty(f"proj{k}__ibx", key, (n * 8,))
         nat.create(f"proj{k}__ibb", np.zeros((proj.pre_pop.size + 31) // 32, dtype=np.uint32))
         if proj.plastic:
-            nat.create_empty(f"proj{k}__pv", np.float64, (nnz,))
+            nat.create_empty(f"proj{k}__pv", np.float64, (lay["nnz"],))
+        # spikes are counted in every `step`-th word (at most 511 atomics per step)
+        words = lay["w1"] - lay["w0"]
+        span = (lay["w0"], lay["w1"], max(1, words // 256))
+        ranges = self.activity.setdefault(pre, [])
+        if span not in ranges:
+            ranges.append(span)
+        lay["act"] = ranges.index(span)
+        # Rows are walked when a neuron expects more than 1.5 events of the step (3
+        # in projections of 4M synapses and more): beyond, inboxes run over here and
+        # there, and the walk of every row by the whole GPU costs less. us per step,
+        # inboxes and rows: 4000 neurons with 200 synapses each, 2 events 8.2 and
+        # 7.9; 1000 with 1000, 2 events 6.6 and 8.9, 10 events 104 and 11 (207 with
+        # overflowing rows walked one by one, 14.5 by a kernel that always walks);
+        # 100,000 with 500, 2 events 44 and 127, 5 events 208 and 150.
+        # A neuron of long rows among short ones counts with half its row if four
+        # of a warp's have them (up to three the warp walks without delay).
+        by_post = np.zeros(-(-n // 32) * 32)
+        by_post[posts] = lengths
+        fourth = np.partition(by_post.reshape(-1, 32), 28, axis=1)[:, 28].max()
+        length = max(lay["nnz"] / max(1, np.count_nonzero(lengths)), fourth / 2)
+        events = 1.5 if lay["nnz"] < 4_000_000 else 3.0
+        steps = 1 if proj._delay_steps is None else self.slots[pre]
+        lay["dense"] = int(events * steps * -(-words // span[2]) * 32 / max(length, 1e-9))
 
     def _create_delays(self, proj):
         k = proj.id
@@ -925,7 +961,7 @@ class CompiledNetwork:
                 row_of = np.full(proj.post_pop.size, -1, dtype=np.int32)
                 row_of[post_rank] = np.arange(rows, dtype=np.int32)
                 nat.create(f"proj{k}__row_of", row_of)
-            self._create_inbox(proj, nnz)
+            self._create_inbox(proj, lay, post_rank, np.diff(row_ptr))
             # warp per post row: exact order, per-synapse delays, and plastic
             # delayed projections (the spike lists hold only the last step)
             gather = self.exact or proj._delay_steps is not None or (

@@ -1000,7 +1000,9 @@ __device__ __forceinline__ void anb_spike_gather_delayed(int n_rows, const int* 
 // bounds of a word's columns by a thread per neuron, the first two 13.8 and 9.6
 // us; with the entries of all inboxes of a thread fetched at once, 11.4 and 9.6;
 // with a plastic synapse's place in the inbox asked for before its statements,
-// 8.4 for the plastic one.
+// 8.4 for the plastic one. Steps with many spikes overfill the inboxes; then all
+// rows are walked (the update kernels count spikes for this decision, which costs
+// 0.1 to 0.5 us per step).
 #define ANB_INBOX 8          // entries per post neuron: one 32-byte sector of 32-bit keys
 #define ANB_DELIVER_WORDS 32 // bitmap words per CTA of a deliver kernel, at most
 #define ANB_DELIVER_LIST (32 * ANB_DELIVER_WORDS)
@@ -1095,6 +1097,16 @@ __device__ __forceinline__ void anb_for_spikes(const int* list, int n, Body body
   }
 }
 
+// Spikes counted in the steps before t whose slots the ring holds (every step
+// but t itself; the calling warp).
+__device__ __forceinline__ anb_u32 anb_activity(const anb_u32* ring, int slots, long long t) {
+  const int now = anb_ring_slot(t, slots);
+  anb_u32 n = 0u;
+  for (int q = threadIdx.x & 31; q < slots; q += 32)
+    if (q != now) n += ring[q];
+  return __reduce_add_sync(0xffffffffu, n);
+}
+
 // Appends `key` to the inbox of neuron `post` (entries beyond ANB_INBOX are
 // only counted: the neuron then walks its row).
 template <typename K>
@@ -1156,49 +1168,138 @@ __device__ __forceinline__ void anb_inbox_first(const unsigned long long* __rest
   b = e.y;
 }
 
-// g plus the weights w[j] of the row's synapses whose pre neuron's bit is set,
-// in ascending pre rank (whole warp, one row).
-template <typename R>
+// Rows walked in the reference's order: the conductance g plus the weights w[j] of
+// the row's synapses whose pre neuron's bit is set, in ascending pre rank. Loads of
+// U steps are issued together, so that a long row is not a chain of trips to L2.
+// (All rows walked, 1000 neurons with 1000 synapses each, 5 % spiking: U = 4, 2, 1
+// 11.2, 13.1, 18.7 us per step; a kernel of its own without U 18.5. The update
+// kernels, where few neurons' inboxes run over, take U = 1: with more in flight
+// their other code slowed down, 11.9 instead of 11.6 us per step of 100,000 neurons
+// with 500 synapses each.) Whole warp, one row. Not inlined: half the compile time.
+template <typename R, int U>
 __device__ __noinline__ R anb_row_gather(R g, int beg, int end, const int* __restrict__ col,
-                                            const R* __restrict__ w, const anb_u32* bits) {
+                                         const R* __restrict__ w, const anb_u32* bits) {
   const int lane = threadIdx.x & 31;
-  for (int base = beg; base < end; base += 32) {
-    const int j = base + lane;
-    const bool sp = j < end && anb_bit(bits, col[j]);
-    anb_u32 m = __ballot_sync(0xffffffffu, sp);
-    const R wj = sp ? w[j] : R(0);
-    while (m) {
-      const int b = __ffs(m) - 1;
-      m &= m - 1;
-      g += __shfl_sync(0xffffffffu, wj, b);
-    }
+  for (int base = beg; base < end; base += 32 * U) {
+    int c[U];
+    bool sp[U];
+    R v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) c[u] = base + 32 * u + lane < end ? col[base + 32 * u + lane] : -1;
+#pragma unroll
+    for (int u = 0; u < U; ++u) sp[u] = c[u] >= 0 && anb_bit(bits, c[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = sp[u] ? w[base + 32 * u + lane] : R(0);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      for (anb_u32 m = __ballot_sync(0xffffffffu, sp[u]); m; m &= m - 1)
+        g += __shfl_sync(0xffffffffu, v[u], __ffs(m) - 1);
+  }
+  return g;
+}
+
+// One row per lane (lanes on their own): four and more overflowing neurons of a
+// warp. (32 rows of 1000 synapses one after another took 207 us, this way 104.)
+template <typename R>
+__device__ __noinline__ R anb_lane_gather(R g, int beg, int end, const int* __restrict__ col,
+                                          const R* __restrict__ w, const anb_u32* bits) {
+  constexpr int U = 4;
+  for (int base = beg; base < end; base += U) {
+    int c[U];
+    bool sp[U];
+    R v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) c[u] = base + u < end ? col[base + u] : -1;
+#pragma unroll
+    for (int u = 0; u < U; ++u) sp[u] = c[u] >= 0 && anb_bit(bits, c[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = sp[u] ? w[base + u] : R(0);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (sp[u]) g += v[u];
   }
   return g;
 }
 
 // The same with one delay per synapse: emission steps t - slots .. t - 1 in
-// order, ascending pre rank within each. The ring slot of the oldest step is
-// read from its copy `oldest` (the update kernels of step t write that slot).
-template <typename R>
+// order, ascending pre rank within each: one pass over the row for the delays
+// that deliver a spike in step t, then one for each of them. The ring slot of the
+// oldest step is read from `oldest` (the update kernels of step t write that
+// slot: they keep a copy).
+struct anb_delay_ring {
+  const anb_u32 *ring, *oldest;
+  int words, slots, now;                               // now: the slot of step t
+  __device__ __forceinline__ const anb_u32* at(int d) const {
+    return d == slots ? oldest : ring + (size_t)(now - d < 0 ? now - d + slots : now - d) * words;
+  }
+};
+
+template <typename R, int U>
 __device__ __noinline__ R anb_row_gather_delayed(R g, int beg, int end, const int* __restrict__ col,
                                                  const R* __restrict__ w,
-                                                 const int* __restrict__ dly, const anb_u32* ring,
-                                                 const anb_u32* oldest, int words, int slots,
-                                                 long long t) {
+                                                 const int* __restrict__ dly, const anb_delay_ring q) {
   const int lane = threadIdx.x & 31;
-  for (int d = slots; d >= 1; --d) {
-    const anb_u32* bits = d == slots ? oldest : ring + (size_t)anb_ring_slot(t - d, slots) * words;
-    for (int base = beg; base < end; base += 32) {
-      const int j = base + lane;
-      const bool sp = j < end && dly[j] == d && anb_bit(bits, col[j]);
-      anb_u32 m = __ballot_sync(0xffffffffu, sp);
-      const R wj = sp ? w[j] : R(0);
-      while (m) {
-        const int b = __ffs(m) - 1;
-        m &= m - 1;
-        g += __shfl_sync(0xffffffffu, wj, b);
-      }
+  anb_u32 lo = 0u, hi = 0u;                            // the delays that deliver
+  for (int base = beg; base < end; base += 32 * U) {
+    int c[U], d[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int j = base + 32 * u + lane;
+      c[u] = j < end ? col[j] : -1;
+      d[u] = j < end ? dly[j] : 0;
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c[u] >= 0 && anb_bit(q.at(d[u]), c[u])) {
+        if (d[u] < 32) lo |= 1u << d[u];
+        else hi |= 1u << (d[u] - 32);
+      }
+  }
+  lo = __reduce_or_sync(0xffffffffu, lo);
+  hi = __reduce_or_sync(0xffffffffu, hi);
+  for (unsigned long long rest = (unsigned long long)hi << 32 | lo; rest;) {
+    const int at = 63 - __clzll(rest);
+    rest &= ~(1ull << at);
+    const anb_u32* bits = q.at(at);
+    for (int base = beg; base < end; base += 32 * U) {
+      int c[U];
+      bool sp[U];
+      R v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int j = base + 32 * u + lane;
+        c[u] = j < end && dly[j] == at ? col[j] : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) sp[u] = c[u] >= 0 && anb_bit(bits, c[u]);
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = sp[u] ? w[base + 32 * u + lane] : R(0);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        for (anb_u32 m = __ballot_sync(0xffffffffu, sp[u]); m; m &= m - 1)
+          g += __shfl_sync(0xffffffffu, v[u], __ffs(m) - 1);
+    }
+  }
+  return g;
+}
+
+template <typename R>
+__device__ __noinline__ R anb_lane_gather_delayed(R g, int beg, int end, const int* __restrict__ col,
+                                                  const R* __restrict__ w,
+                                                  const int* __restrict__ dly, anb_delay_ring q) {
+  unsigned long long rest = 0ull;
+#pragma unroll 4
+  for (int j = beg; j < end; ++j) {
+    const int d = dly[j];
+    if (anb_bit(q.at(d), col[j])) rest |= 1ull << d;
+  }
+  while (rest) {
+    const int at = 63 - __clzll(rest);
+    rest &= ~(1ull << at);
+    const anb_u32* bits = q.at(at);
+#pragma unroll 4
+    for (int j = beg; j < end; ++j)
+      if (dly[j] == at && anb_bit(bits, col[j])) g += w[j];
   }
   return g;
 }

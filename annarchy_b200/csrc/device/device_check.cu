@@ -62,8 +62,11 @@ extern "C" __global__ void check_inbox(const anb_u32* spk, const int* cp, const 
   const int i = threadIdx.x;
   double s = anb_inbox_add(g[i], cnt[i], ent, i, w);
   s = anb_inbox_add(s, cnt[i], entd, i, w);
-  s = anb_row_gather<double>(s, rp[0], rp[1], c, w, spk);
-  g[i] = anb_row_gather_delayed<double>(s, rp[0], rp[1], c, w, d, spk, spk, 8, 4, 9);
+  s = anb_row_gather<double, 1>(s, rp[0], rp[1], c, w, spk);
+  s = anb_lane_gather<double>(s, rp[i], rp[i + 1], c, w, spk);
+  const anb_delay_ring q = {spk, spk, 8, 4, anb_ring_slot(9, 4)};
+  s = anb_lane_gather_delayed<double>(s, rp[i], rp[i + 1], c, w, d, q);
+  g[i] = anb_row_gather_delayed<double, 4>(s, rp[0], rp[1], c, w, d, q) + anb_activity(cnt, 5, 9);
 }
 extern "C" __global__ void check_spike_scatter(const anb_u32* spk, const int* cp, const int* pi,
                                                const anb_bf16* w, float* g) {

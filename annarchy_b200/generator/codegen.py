@@ -585,6 +585,13 @@ class CodeGenerator:
             stores.append(f"anb_store_tile({self.ptr('tc__xt')} + (size_t){first * copies * 64}, anb_i / {size1}, "
                           f"anb_i % {size1}, {copies}, {rv});")
         ballot = ""
+        counted = ""
+        if grid_path and pop.id in self.c.activity:
+            ring, stride = self.slots(pop) + 1, self.c.activity_stride(k)
+            counted = "".join(f"""
+        if ((threadIdx.x & 31) == 0 && anb_m && anb_i < anb_n && (anb_i >> 5) >= {w0} && (anb_i >> 5) < {w1}{f" && ((anb_i >> 5) - {w0}) % {step} == 0" if step > 1 else ""})
+          atomicAdd({self.ptr(f'pop{k}__nsp')} + {i * stride} + anb_ring_slot(t, {ring}), __popc(anb_m));"""
+                              for i, (w0, w1, step) in enumerate(self.c.activity[pop.id]))
         listed = (spiking and cluster is None and not local_engine and not self.exact
                   and self.c.spike_lists)
         recs = "" if (local_engine or cluster is not None) else self._fused_spike_records(pop)
@@ -613,7 +620,7 @@ class CodeGenerator:
             ballot = f"""
       {{
         const anb_u32 anb_m = __ballot_sync(0xffffffffu, anb_spiked);
-        if ((threadIdx.x & 31) == 0 && {widx} < {lim}) {spk_dst}[{widx} >> 5] = anb_m;{recs}
+        if ((threadIdx.x & 31) == 0 && {widx} < {lim}) {spk_dst}[{widx} >> 5] = anb_m;{recs}{counted}
       }}"""
         nl = "\n        "
         keep, events = self._fused_post_events(pop) if grid_path and spiking else ("", "")
@@ -712,7 +719,8 @@ class CodeGenerator:
         """The step's increments of a neuron's conductances from its inboxes
         (inbox_projections), projection by projection, before its update; a
         neuron whose inbox ran over walks its row (the whole warp, one such
-        neuron at a time). Rewrites the update's loads of those conductances.
+        neuron at a time, or every lane its own where there are four or more).
+        Rewrites the update's loads of those conductances.
         Second, the code that fetches the first two entries of every inbox and
         their weights, all projections (and neurons of the thread) at once:
         one after another they were two dependent trips to L2 per projection."""
@@ -749,13 +757,14 @@ class CodeGenerator:
                 fetch.append(f"anb_ic{k} = {value(f'anb_in_c{k}')};")
                 w = p("pv") if proj.plastic else p("w")
                 rows = f"{p('row_ptr')}[anb_r], {p('row_ptr')}[anb_r + 1], {p('col')}, {w}"
+                late = ""
                 if proj._delay_steps is not None:
                     a = proj.pre_pop
-                    walk = (f"anb_row_gather_delayed<{R}>(anb_g, {rows}, {p('dly')}, "
-                            f"{self.ptr(f'pop{a.id}__spk')}, {p('ibb')}, {(a.size + 31) // 32}, "
-                            f"{self.slots(a)}, t)")
+                    late = "_delayed"
+                    rows += (f", {p('dly')}, anb_delay_ring{{{self.ptr(f'pop{a.id}__spk')}, {p('ibb')}, "
+                             f"{(a.size + 31) // 32}, {self.slots(a)}, anb_ring_slot(t, {self.slots(a)})}}")
                 else:
-                    walk = f"anb_row_gather<{R}>(anb_g, {rows}, {p('ibb')})"
+                    rows += f", {p('ibb')}"
                 short = ""
                 if early:
                     key = "unsigned long long" if proj._delay_steps is not None else "anb_u32"
@@ -774,11 +783,20 @@ class CodeGenerator:
                 work.append(f"""{short}
           if (anb_ic{k} && anb_ic{k} <= ANB_INBOX)
             anb_gd_{T} = anb_inbox_add(anb_gd_{T}, anb_ic{k}, {p('ibx')}, anb_i, {w});
-          for (anb_u32 anb_m = __ballot_sync(0xffffffffu, anb_ic{k} > ANB_INBOX); anb_m; anb_m &= anb_m - 1) {{
-            const int anb_l = __ffs(anb_m) - 1;
+          anb_u32 anb_o{k} = __ballot_sync(0xffffffffu, anb_ic{k} > ANB_INBOX);
+          if (__popc(anb_o{k}) > 3) {{
+            if (anb_ic{k} > ANB_INBOX) {{
+              const int anb_r = {p('row_of')}[anb_i];
+              anb_gd_{T} = anb_lane_gather{late}<{R}>(anb_gd_{T}, {rows});
+            }}
+            __syncwarp();
+            anb_o{k} = 0u;
+          }}
+          for (; anb_o{k}; anb_o{k} &= anb_o{k} - 1) {{
+            const int anb_l = __ffs(anb_o{k}) - 1;
             const {R} anb_g = __shfl_sync(0xffffffffu, anb_gd_{T}, anb_l);
             const int anb_r = {p('row_of')}[__shfl_sync(0xffffffffu, anb_i, anb_l)];
-            const {R} anb_s = {walk};
+            const {R} anb_s = anb_row_gather{late}<{R}, 1>(anb_g, {rows});
             if ((threadIdx.x & 31) == anb_l) anb_gd_{T} = anb_s;
           }}""")
                 clear.append(f"if (anb_ic{k}) {p('ibn')}[anb_i] = 0u;")
@@ -1800,8 +1818,19 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) proj{k}_psp() {{
         to the post neurons' inboxes; a plastic projection runs its pre-spike
         statements and keeps the transmitted value per synapse (pv). The words
         the update kernels may overwrite are copied for the neurons that will
-        walk their rows."""
+        walk their rows.
+
+        After steps with many spikes (lay["dense"], by the counts the update
+        kernels keep) a target's projections are walked row by row instead, by
+        all blocks: a warp per post neuron adds what its synapses transmit, in
+        order, to the conductance itself."""
+        # (known when all projections have been seen: loads of the counts, the bits)
+        ASK, MODE = "/*ask*/", "/*mode*/"
         parts, first = [], 0
+        groups: dict = {}
+        for proj in projs:
+            groups.setdefault((proj.post_pop.id, proj.target), []).append(proj)
+        group_of = {q.id: i for i, v in enumerate(groups.values()) for q in v}
         for proj in projs:
             k, a = proj.id, proj.pre_pop
             lay = self.c.layout[k]
@@ -1824,17 +1853,22 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) proj{k}_psp() {{
             decl = ""
             now = f"""{ENTER}
       const long long t = *{self.ptr('t')};"""
+            rows_instead = f"(anb_mode >> {group_of[k]} & 1u)"
+            ask = f"{ASK}\n      {MODE}"
             find = f"""const int anb_ns = anb_list_spikes(anb_list, {bits} + {lay['w0']}, {(a.size + 31) // 32}, {lay['w0']}, {words}, {slots}, t,
-                                         anb_w, anb_nw, {p('col_ptr')}, nullptr);"""
+                                         anb_w, {rows_instead} ? 0 : anb_nw, {p('col_ptr')}, nullptr);"""
             if not slots and per * 32 <= BLOCK:
                 # a thread per neuron: the column's bounds before the wait
                 now = f"""const int anb_id = ({lay['w0']} + anb_w) * 32 + (int)threadIdx.x;
       const bool anb_in = (int)threadIdx.x < anb_nw * 32 && anb_id < {a.size};
       const int anb_pb = anb_in ? {p('col_ptr')}[anb_id] : 0, anb_pe = anb_in ? {p('col_ptr')}[anb_id + 1] : 0;
       {now}"""
-                find = f"""const anb_u32* anb_bits = {bits};
-      const int anb_ns = anb_list_ranges(anb_list, ((int)threadIdx.x & 31) < anb_nw ? anb_bits[{lay['w0']} + anb_w + (threadIdx.x & 31)] : 0u,
-                                         anb_id, anb_pb, anb_pe);"""
+                ask = f"""const anb_u32* anb_bits = {bits};
+      const anb_u32 anb_word = ((int)threadIdx.x & 31) < anb_nw ? anb_bits[{lay['w0']} + anb_w + (threadIdx.x & 31)] : 0u;
+      {ASK}"""
+                find = f"""int anb_ns = anb_list_ranges(anb_list, anb_word, anb_id, anb_pb, anb_pe);
+      {MODE}
+      if {rows_instead} anb_ns = 0;"""
             if proj.plastic:
                 stmts = self._event_driven(proj, "j", "t-1") + self.syn_spike_statements(proj, "pre_spike")
                 body = "\n          ".join(stmts)
@@ -1860,6 +1894,7 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) proj{k}_psp() {{
       const int anb_nw = min({per}, {words * max(1, slots)} - anb_w);
       {decl}
       {now}
+      {ask}
       const anb_u32* anb_old = {oldest};
       for (int q = (int)blockIdx.x - {first}; q < {-(-words // BLOCK)}; q += {ctas}) {{
         const int anb_cw = q * {BLOCK} + threadIdx.x;
@@ -1872,14 +1907,118 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) proj{k}_psp() {{
         }});
     }}""")
             first += ctas
+        modes, walks, neurons, early = [], [], 1, ""
+        for i, group in enumerate(groups.values()):
+            many = []
+            for proj in group:
+                a, lay = proj.pre_pop, self.c.layout[proj.id]
+                ring, stride = self.slots(a) + 1, self.c.activity_stride(a.id)
+                at = lay["act"] * stride
+                count = f"{self.ptr(f'pop{a.id}__nsp')} + {at}"
+                if proj._delay_steps is not None or ring == 2:
+                    # (asked for with the bitmap's words)
+                    early += f"""
+      const uint2 anb_n{proj.id} = *reinterpret_cast<const uint2*>({count}{f' + {stride - 2}' if ring > 2 else ''});"""
+                    count = f"(t & 1 ? anb_n{proj.id}.{'y' if ring > 2 else 'x'} : anb_n{proj.id}.{'x' if ring > 2 else 'y'})"
+                else:
+                    d = f"{self.ptr(f'proj{proj.id}__delay')}[0]" if self.delayed(proj) else "1"
+                    early += f"""
+      const anb_u32 anb_n{proj.id} = ({count})[anb_ring_slot(t - {d}, {ring})];"""
+                    count = f"anb_n{proj.id}"
+                many.append(f"{count} > {lay['dense']}u")
+            modes.append(f"(({' || '.join(many)}) ? {1 << i}u : 0u)")
+            walks.append(self._walk_rows(i, group))
+            neurons = max(neurons, group[0].post_pop.size)
+        # the counter of this step starts; the sum over the history for the next
+        # step (which will not see this step's spikes: those of delay 1)
+        keep = ""
+        for a, ranges in self.c.activity.items():
+            ring, stride, n = self.c.slots[a] + 1, self.c.activity_stride(a), self.ptr(f"pop{a}__nsp")
+            for i in range(len(ranges)):
+                keep += f"""
+      if (threadIdx.x == 0) {n}[{i * stride} + anb_ring_slot(t, {ring})] = 0u;"""
+                if ring > 2:
+                    keep += f"""
+      {{
+        const anb_u32 anb_sum = anb_activity({n} + {i * stride}, {ring}, t);
+        if (threadIdx.x == 0) {n}[{(i + 1) * stride - 2} + (int)((t + 1) & 1)] = anb_sum;
+      }}"""
+        mode = " | ".join(modes)
+        # blocks for the rows (three per SM at most; in other steps those beyond
+        # the bitmaps' have nothing to do but the first, which keeps the counts)
+        ctas = max(first + 1, min(444, -(-neurons * 32 // BLOCK)))
+        rest = f"""
+    if ((int)blockIdx.x >= {first}) {{
+      {ENTER}
+      const long long t = *{self.ptr('t')};
+{early}
+      anb_mode = {mode};
+      if ((int)blockIdx.x == {first} && threadIdx.x < 32) {{{keep}
+      }}
+    }}"""
+        parts = [part.replace(ASK, early).replace(MODE, f"anb_mode = {mode};") for part in parts]
         name = "anb_deliver"
         return f"""
 extern "C" __global__ void __launch_bounds__({BLOCK}) {name}() {{
     const {self.real} dt = ({self.real})(*{self.ptr('dt')});
     __shared__ int anb_list[4 * ANB_DELIVER_LIST + 1];
-    {''.join(parts)}
+    // bit i: the rows of the i-th target are walked
+    anb_u32 anb_mode = 0u;
+    {''.join(parts)}{rest}
+    if (anb_mode) {{
+      const long long t = *{self.ptr('t')};{''.join(walks)}
+    }}
 }}
-""", (name, first, BLOCK, 0)
+""", (name, ctas, BLOCK, 0)
+
+    def _walk_rows(self, i: int, group) -> str:
+        """The transmissions of one target's projections, a warp per post
+        neuron (deliver_kernel)."""
+        R, post = self.real, group[0].post_pop
+        g = self.ptr(f"pop{post.id}__g_{group[0].target}")
+        adds, rows = [], ""
+        for proj in group:
+            a, k = proj.pre_pop, proj.id
+            p = lambda n, k=k: self.ptr(f"proj{k}__{n}")
+            rows += f"""
+        const int anb_r{k} = {p('row_of')}[anb_i];"""
+            row = f"{p('row_ptr')}[anb_r{k}], {p('row_ptr')}[anb_r{k} + 1], {p('col')}" + ("" if proj.plastic else f", {p('w')}")
+            if proj.plastic:
+                body = "\n            ".join(self._event_driven(proj, "j", "t-1")
+                                            + self.syn_spike_statements(proj, "pre_spike"))
+                known = " ".join(f"const {ct} {n} = {src}[0];" for ct, n, src in self._constants(proj))
+                add = f"""{self._syn_arrays(proj)}
+          {known}
+          const anb_u32* anb_bits = {self.pre_spk(proj)};
+          for (int anb_b = {p('row_ptr')}[anb_r{k}], anb_e = {p('row_ptr')}[anb_r{k} + 1]; anb_b < anb_e; anb_b += 32) {{
+            const int j = anb_b + anb_lane;
+            const bool anb_sp = j < anb_e && anb_bit(anb_bits, {p('col')}[j]);
+            {R} sum = ({R})0;
+            if (anb_sp) {{
+            {self.syn_index_defs(body, f"{p('col')}[j]", "anb_i")}{body}
+            }}
+            for (anb_u32 anb_m = __ballot_sync(0xffffffffu, anb_sp); anb_m; anb_m &= anb_m - 1)
+              anb_g += __shfl_sync(0xffffffffu, sum, __ffs(anb_m) - 1);
+          }}"""
+            elif proj._delay_steps is not None:
+                words, slots, spk = (a.size + 31) // 32, self.slots(a), self.ptr(f"pop{a.id}__spk")
+                add = f"""const int anb_slot = anb_ring_slot(t, {slots});
+          anb_g = anb_row_gather_delayed<{R}, 4>(anb_g, {row}, {p('dly')},
+                                           anb_delay_ring{{{spk}, {spk} + (size_t)anb_slot * {words}, {words}, {slots}, anb_slot}});"""
+            else:
+                add = f"anb_g = anb_row_gather<{R}, 4>(anb_g, {row}, {self.pre_spk(proj)});"
+            adds.append(f"""
+        if (anb_r{k} >= 0) {{  // {proj.name}
+          {add}
+        }}""")
+        return f"""
+      if (anb_mode >> {i} & 1u) {{  // population {post.name}, g_{group[0].target}
+      const int anb_lane = threadIdx.x & 31, anb_step = (int)(gridDim.x * blockDim.x) >> 5;
+      for (int anb_i = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; anb_i < {post.size}; anb_i += anb_step) {{
+        {R} anb_g = {g}[anb_i];{rows}{''.join(adds)}
+        if (anb_lane == 0) {g}[anb_i] = anb_g;
+      }}
+      }}"""
 
     def fused_transmissions(self, projs) -> tuple[str, tuple]:
         """One launch for the transmissions that only add with atomics: the
