@@ -654,6 +654,12 @@ class CodeGenerator:
       }}
     }}"""
         first = 0
+        # neurons of a CTA and pass, and the thread's one (fewer than threads where
+        # the post events of few neurons occupy the whole CTA)
+        span, mine = "blockDim.x", "{} + threadIdx.x"
+        if keep and self.update_span(pop) < BLOCK:
+            span = str(self.update_span(pop))
+            mine = f"((int)threadIdx.x < {span} ? {{}} + (int)threadIdx.x : anb_n)"
         if grid_path and (K > 1 or drain):
             if pop.id in getattr(self.c, "owned", {}):
                 first, size = self.c.owned[pop.id]
@@ -667,20 +673,20 @@ class CodeGenerator:
     {{  // population {pop.name}: update{' and spike gather' if spiking else ''}, {K} neurons per
         // thread and pass with all their loads issued first
       const int anb_n = {size if size is not None else pop.size};{shared}
-      for (int anb_base0 = {first} + blockIdx.x * blockDim.x * {K}; anb_base0 < anb_n;
-           anb_base0 += gridDim.x * blockDim.x * {K}) {{{events_pre % "anb_base0"}
+      for (int anb_base0 = {first} + blockIdx.x * {span} * {K}; anb_base0 < anb_n;
+           anb_base0 += gridDim.x * {span} * {K}) {{{events_pre % "anb_base0"}
         {arrays}
 #pragma unroll
         for (int anb_k = 0; anb_k < {K}; ++anb_k) {{
-          const int anb_j = anb_base0 + anb_k * blockDim.x + threadIdx.x;
+          const int anb_j = {mine.format(f"anb_base0 + anb_k * {span}")};
           if (anb_j < anb_n) {{
           {fetch}
           }}
         }}{entries}
 #pragma unroll
         for (int anb_k = 0; anb_k < {K}; ++anb_k) {{
-        const int anb_base = anb_base0 + anb_k * blockDim.x;
-        const int anb_i = anb_base + threadIdx.x;
+        const int anb_base = anb_base0 + anb_k * {span};
+        const int anb_i = {mine.format("anb_base")};
         bool anb_spiked = false;{drain}
         if (anb_i < anb_n) {{
         {unpack}
@@ -698,13 +704,13 @@ class CodeGenerator:
             # a sharded network updates the owned slice [first, anb_n) only
             if grid_path and pop.id in getattr(self.c, "owned", {}):
                 first, size = self.c.owned[pop.id]
-            loop = (f"for (int anb_base = {first} + blockIdx.x * blockDim.x; anb_base < anb_n; "
-                    "anb_base += gridDim.x * blockDim.x)")
+            loop = (f"for (int anb_base = {first} + blockIdx.x * {span}; anb_base < anb_n; "
+                    f"anb_base += gridDim.x * {span})")
         return f"""
     {{  // population {pop.name}: update{' and spike gather' if spiking else ''}
       const int anb_n = {size if size is not None else pop.size};{shared}
       {loop} {{{events_pre % "anb_base"}
-        const int anb_i = anb_base + threadIdx.x;
+        const int anb_i = {mine.format("anb_base")};
         bool anb_spiked = false;{drain}
         if (anb_i < anb_n) {{
         {nl.join(loads)}
@@ -2073,8 +2079,24 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) anb_transmit() {{{''.join(
         their own deals them out. 20,000 neurons 10.1 -> 7.5 us per step with
         the fused form, 60,000 10.5 (own kernel) and 10.7, 200,000 13.1 and
         15.7, 1M 24.6 and 29.6."""
-        return (self.fuse and self.own_post_events(proj)
-                and self.neurons_per_thread(proj.post_pop) == 1)
+        if not (self.fuse and self.own_post_events(proj) and self.neurons_per_thread(proj.post_pop) == 1):
+            return False
+        # (single precision, whose own kernel deals out pieces of rows: not with
+        # few CTAs for long rows. 1000 neurons of 1000 synapses each, 50 of them
+        # spiking 27.6 us, own kernel 14.8; 0.2 spiking 4.3 and 4.4. Double 101, 104.)
+        lay = self.c.layout[proj.id]
+        return self.exact or proj.post_pop.size >= 32 * 148 or lay["nnz"] <= 256 * lay["rows"]
+
+    def update_span(self, pop) -> int:
+        """Neurons per CTA of a population's update kernel: with post events in
+        it so few that the events of a step with many spikes still spread over
+        the SMs (all of a CTA's warps take part in them). 256
+        neurons per CTA, a step with 5 % of 1000 neurons of 1000 plastic synapses
+        each: 687 us in double precision, 101 with 32 per CTA (single: 66 and 28)."""
+        if not any(p.post_pop is pop and self.post_fused(p) for p in self.net.projections):
+            return BLOCK
+        lo, hi = getattr(self.c, "owned", {}).get(pop.id, (0, pop.size))
+        return 32 * max(1, min(BLOCK // 32, -(-(hi - lo) // 32) // 148))
 
     def _post_args(self, proj) -> list:
         return [p["name"] for p in proj.desc["parameters"] + proj.desc["variables"]
@@ -2156,7 +2178,9 @@ __device__ __noinline__ anb_tr{k} proj{k}_post_syn(anb_tr{k} anb_s, const long l
             first, n = self.c.owned[pop.id]
         projs = [p for p in self.net.projections if p.post_pop is pop and self.post_fused(p)]
         if projs:
-            out.append(f"const int anb_i0 = {first} + blockIdx.x * blockDim.x + threadIdx.x;")
+            span = self.update_span(pop)
+            out.append(f"const int anb_i0 = {first} + blockIdx.x * {span} + threadIdx.x;" if span == BLOCK else
+                       f"const int anb_i0 = (int)threadIdx.x < {span} ? {first} + (int)blockIdx.x * {span} + (int)threadIdx.x : {n};")
         for proj in projs:
             k = proj.id
             p = lambda n, k=k: self.ptr(f"proj{k}__{n}")
@@ -2415,7 +2439,8 @@ extern "C" __global__ void __launch_bounds__({PERSISTENT_BLOCK}, 1) anb_grid_run
                 kernels.append(self.pop_kernel(pop))
                 lo, hi = getattr(self.c, "owned", {}).get(pop.id, (0, pop.size))
                 K = self.neurons_per_thread(pop)
-                plan.append((f"pop{pop.id}_step", grid_for(max(1, -(-(hi - lo) // K))), BLOCK, 0))
+                blocks = max(1, -(-(hi - lo) // self.update_span(pop))) if K == 1 else 0
+                plan.append((f"pop{pop.id}_step", blocks or grid_for(max(1, -(-(hi - lo) // K))), BLOCK, 0))
             if pop._globalops:
                 kernels.append(self.globalops_kernel(pop))
                 plan.append((f"pop{pop.id}_globalops", 1, 32 if self.exact else 1024, 0))
