@@ -636,6 +636,7 @@ class CodeGenerator:
         nl = "\n        "
         keep, events = self._fused_post_events(pop) if grid_path and spiking else ("", "")
         if keep:
+            assert ballot.count("__ballot_sync(0xffffffffu, anb_spiked);") == 1
             ballot = ballot.replace("__ballot_sync(0xffffffffu, anb_spiked);",
                                     "__ballot_sync(0xffffffffu, anb_spiked);" + keep.replace("anb_mw", "anb_m"), 1)
             events_pre = """
@@ -2060,6 +2061,7 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) {name}() {{
         for proj in projs:
             n = self.c.layout[proj.id]["grid"]
             src = self.spike_kernel(proj)
+            assert src.count('extern "C"') == 1 and "return;" not in src, proj.name
             body = src[src.index("{") + 1:src.rindex("}")]
             body = body.replace("(int)blockIdx.x", "anb_blk").replace("(int)gridDim.x", "anb_nblk")
             body = body.replace("blockIdx.x", "anb_blk").replace("gridDim.x", "anb_nblk")

@@ -566,7 +566,8 @@ extern "C" __global__ void __launch_bounds__({block}, 1) anb_cluster_run(long lo
         code = gen.neuron_update(pop, local_engine=True, smem=smem, cluster={}, ballot_hook=hook)
         code = f"{{ {gen._scoped_globals(pop)[1]}{code}}}"
         code = re.sub(r"(anb_rg\d+_\w+)\[anb_q\]", r"\1", code)
-        code = code.replace("for (int anb_q0 = 0; anb_q0 < anb_cnt; anb_q0 += blockDim.x) {",
-                            "{ const int anb_q0 = 0;")
-        return code.replace(f"const int anb_base = anb_base{k}, anb_cnt = anb_cnt{k};",
-                            f"const int anb_base = anb_base{k}, anb_cnt = anb_cnt{k}; (void)anb_base;")
+        # one pass over the CTA's neurons, whose state is a register each
+        loop = "for (int anb_q0 = 0; anb_q0 < anb_cnt; anb_q0 += blockDim.x) {"
+        names = f"const int anb_base = anb_base{k}, anb_cnt = anb_cnt{k};"
+        assert code.count(loop) == code.count(names) == 1 and not re.search(r"anb_rg\d+_\w+\[", code)
+        return code.replace(loop, "{ const int anb_q0 = 0;").replace(names, names + " (void)anb_base;")
