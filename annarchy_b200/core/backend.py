@@ -44,6 +44,10 @@ def from_bf16(h: np.ndarray) -> np.ndarray:
     return (np.asarray(h, dtype=np.uint32) << 16).view(np.float32).astype(np.float64)
 
 
+class NoCluster(RuntimeError):
+    """A spiking network that fits no cluster of the device."""
+
+
 class CompiledNetwork:
     def __init__(self, net, dry: bool = False):
         self.net = net
@@ -270,10 +274,9 @@ class CompiledNetwork:
         nat = self.native
         masks, self.masks = self.masks, None
         if self.engine == "cluster":
-            self._build_cluster_lists()
-            masks.free_arrays()
-            return
-        self._build_plan()
+            self._cluster_lists_or_plan()
+        else:
+            self._build_plan()
         masks.free_arrays()
         t = nat.get_time()
         for pop in self.net.populations:
@@ -300,7 +303,23 @@ class CompiledNetwork:
             self.masks = masks
             self.engine = "cluster"
             return
-        self._build_cluster_lists()
+        if self.net._config.get("engine", "auto") == "local":
+            self._build_cluster_lists()
+        else:
+            self._cluster_lists_or_plan()
+
+    def _cluster_lists_or_plan(self):
+        """The cluster kernel with synapse lists, or, for a network whose lists
+        fit no cluster, the launch plan (transmitting from the bitmaps)."""
+        try:
+            self._build_cluster_lists()
+        except NoCluster:
+            for proj in self.net.projections:
+                for name in ("cl_ptr", "cl_base", "cl_post", "cl_w", "cl_wi", "cl_pal"):
+                    if f"proj{proj.id}__{name}" in self.native.arrays:
+                        self.native.free(f"proj{proj.id}__{name}")
+            self.engine = "grid"
+            self._build_plan()
 
     def _build_cluster_lists(self):
         """The cluster kernel whose CTAs hold lists of their synapses."""
@@ -322,9 +341,9 @@ class CompiledNetwork:
                     self.native.create(f"proj{k}__{name}", arr)
             gen = CodeGenerator(self)
             mod = gen.cluster_module()
+            self.native.load_module(mod.source, mod.options)
+            self.write_constants()
             try:
-                self.native.load_module(mod.source, mod.options)
-                self.write_constants()
                 self.native.set_local_kernel(*mod.local)
             except BackendError as exc:
                 last_err = exc
@@ -332,7 +351,7 @@ class CompiledNetwork:
             self.module = mod
             self.engine = "cluster"
             return
-        raise RuntimeError(f"no cluster configuration fits this network ({last_err})")
+        raise NoCluster(f"no cluster configuration fits this network ({last_err})")
 
     def _write_cluster_weights(self, proj):
         """The weights set after compile() into the cluster kernel's synapse
@@ -348,7 +367,7 @@ class CompiledNetwork:
             n = lay["proj"][k]["pal"][1]
             table = np.unique(w)
             if table.size > n:
-                self._build_cluster_lists()
+                self._cluster_lists_or_plan()
                 return
             self.native.write(f"proj{k}__cl_wi", np.searchsorted(table, w).astype(np.uint8))
             table = np.concatenate([table, np.zeros(n - table.size)])

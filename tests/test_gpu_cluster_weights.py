@@ -91,3 +91,41 @@ def test_weights_set_between_runs(form, kinds, precision):
         else:
             assert x.max() > 0.0
             np.testing.assert_allclose(x, y, rtol=3 * 64 * 2.0**-24, atol=1e-7)
+
+
+def _dense(engine, weights):
+    net = ann.Network(dt=0.1, seed=0)
+    net.config(precision="double", engine=engine)
+    A = net.create(2000, wl.coba_neuron(dict(wl.COBA_PARAMS, I=35.0)))
+    rng = np.random.default_rng(2)
+    m = wl.bernoulli_csr_skip(rng, 2000, 2000, 0.5, 0.002)
+    if weights:
+        m.data *= rng.uniform(0.5, 1.5, m.nnz)
+    p = net.connect(A, A, "exc")
+    p.from_sparse(wl.to_from_sparse(m))
+    A.v = rng.uniform(-60.0, -50.0, 2000)
+    net.compile()
+    return net, A, p, m
+
+
+@pytest.mark.parametrize("weights", [False, True])
+def test_lists_that_fit_no_cluster(weights):
+    """One weight: the mask kernel, and the plan when the weights become
+    different; different weights from the start: the plan, unless the cluster
+    was asked for."""
+    out = []
+    for engine in ("grid", "auto"):
+        net, A, p, m = _dense(engine, weights)
+        assert net.engine == ("cluster" if engine == "auto" and not weights else "grid")
+        net.simulate_steps(40)
+        p.w = list(np.split(np.random.default_rng(5).uniform(0.001, 0.003, m.nnz), np.cumsum(p.dendrite_sizes())[:-1]))
+        assert net.engine == "grid"
+        net.simulate_steps(60)
+        out.append([A.v, A.g_exc])
+        net.close()
+    assert out[0][1].max() > 0.0
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+    if weights:
+        with pytest.raises(RuntimeError):
+            _dense("local", True)
