@@ -51,9 +51,9 @@ UNIT = "GSynOps/s"
 WORKLOAD = "coba_lif_4000_p0.02_dt0.1_10000steps_seed42"
 MODEL_STEPS = 10000
 # DRAM bytes (read + write) per launch of the bench's dominant kernel, from one
-# ncu capture of the same command (dram__bytes_read.sum + dram__bytes_write.sum),
-# keyed by (kernel, precision)
-NCU_TRAFFIC = {("anb_cluster_run", "float"): 1.193472e6, ("anb_cluster_run", "double"): 1.602304e6}
+# ncu capture of runs of the same network and length (dram__bytes_read.sum +
+# dram__bytes_write.sum), keyed by (kernel, precision)
+NCU_TRAFFIC = {("anb_cluster_run", "float"): 2.1468e6, ("anb_cluster_run", "double"): 2.1975e6}
 
 
 def dist_env():
