@@ -390,8 +390,9 @@ __device__ __forceinline__ float anb_w1(const anb_bf16* w) { return anb_bf16_to_
 // Sub-warp per row with 16-byte vector loads of the column indices and
 // weights (streaming, evict-first) over the 4-aligned body of every row and
 // scalar loads at its ends. `rows` (optional) lists the rows to process
-// (row-length binning); `n_rows` is its length.
-template <int G, typename W>
+// (row-length binning); `n_rows` is its length. SET: nothing else is added to
+// these sums (a store does not wait for the old value).
+template <int G, typename W, bool SET = false>
 __device__ __forceinline__ void anb_rate_csr_vec(int n_rows, const int* __restrict__ rows,
                                                  const int* __restrict__ row_ptr,
                                                  const int* __restrict__ col,
@@ -432,7 +433,10 @@ __device__ __forceinline__ void anb_rate_csr_vec(int n_rows, const int* __restri
     for (int j = j0 + 4 * nv + lane; j < end; j += G) s += __ldg(&x[anb_ls_i(&col[j])]) * anb_w1(&w[j]);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, G);
-    if (lane == 0 && row >= 0) sum[post_rank ? post_rank[row] : row] += s;
+    if (lane == 0 && row >= 0) {
+      float* const to = &sum[post_rank ? post_rank[row] : row];
+      *to = SET ? s : *to + s;
+    }
   }
 }
 

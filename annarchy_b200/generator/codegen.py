@@ -540,7 +540,6 @@ class CodeGenerator:
                 for q, part in enumerate(parts):
                     loads.append(f"const {self.real} anb_sum{q}_{t} = {part}[anb_i];")
                     hoist.append((f"const {self.real}", f"anb_sum{q}_{t}", part))
-                    stores.append(f"{part}[anb_i] = ({self.real})0;")
                 if parts:
                     loads.append(f"const {self.real} _sum_{t} = {name}" + "".join(
                         f" + anb_sum{q}_{t}" for q in range(len(parts))) + ";")
@@ -1333,8 +1332,8 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) pop{k}_delay() {{
         0.8M CSR synapses: 13.9 -> 12.2 us per step; 20,000 neurons, 6.0M and
         0.6M: 13.8 -> 11.8; 38,000, 3.8M and 1.8M: 16.7 -> 14.8. The launch adds
         to a target's sums in no order of projections: one that shares them with
-        the panelled projection or another partner writes sums of its own, which
-        the update adds (as many additions, in the projections' order)."""
+        any other projection stores sums of its own, which the update adds (as
+        many additions, in the projections' order)."""
         def static(p):
             return (p.synapse_type.type == "rate" and getattr(p, "_batched", None) is None
                     and not self.rate_learning(p) and not self.custom_psp(p) and not self.delayed(p)
@@ -1347,17 +1346,14 @@ extern "C" __global__ void __launch_bounds__({BLOCK}) pop{k}_delay() {{
         if host is None:
             return out
         room = lay[host.id]["nnz"] // 2
-        written = {(host.post_pop.id, host.target)}
         for q in self.net.projections:
             if static(q) and lay[q.id].get("format") == "csr" and not lay[q.id].get("heavy") and \
                     lay[q.id]["idx_t"] == "int" and lay[q.id]["nnz"] <= room and self.has_update(q.post_pop):
                 out.setdefault(host, []).append(q)
                 room -= lay[q.id]["nnz"]
-                key = (q.post_pop.id, q.target)
-                if key in written:
+                if any(p is not q and p.post_pop is q.post_pop and p.target == q.target for p in self.net.projections):
                     self.c.native.create(f"proj{q.id}__ps", np.zeros(q.post_pop.size, dtype=self.c.real))
-                    self.partner_sums.setdefault(key, []).append(f"proj{q.id}__ps")
-                written.add(key)
+                    self.partner_sums.setdefault((q.post_pop.id, q.target), []).append(f"proj{q.id}__ps")
         return out
 
     def rate_kernel(self, proj, also=()):
@@ -1419,7 +1415,7 @@ extern "C" __global__ void __launch_bounds__({bounds}) {nm}() {{
                 sums = f"proj{q.id}__ps" if f"proj{q.id}__ps" in self.c.native.arrays else f"pop{q.post_pop.id}___sum_{q.target}"
                 call += f"""
     // {q.name}
-    anb_rate_csr_vec<{lq['vgroup']}, {self.c.wctype}>({lq['rows']}, nullptr, {pq('row_ptr')},
+    anb_rate_csr_vec<{lq['vgroup']}, {self.c.wctype}, true>({lq['rows']}, nullptr, {pq('row_ptr')},
         {pq('col')}, {pq('w')}, {self.pre_rate(q)}, {pq('post_rank')}, {self.ptr(sums)});"""
             B = lay["pc_block"]
             return (kern(name, call, B, lay["pc_resident"]),
